@@ -213,6 +213,7 @@ struct ProfDesc {
     u32 qspec;       // speculative threshold (0: none); exact if the best run reaches it
     u32 tpref;       // preferred anchor stages (sparse filter)
     u32 req;         // serving: the request slot this profile belongs to
+    u32 grouped;     // 1: filtered in a group of 32 (group.cuh), no planes of its own
 };
 
 // device-written per-profile results

@@ -18,6 +18,7 @@
 #include "dense.cuh"
 #include "table.cuh"
 #include "sparse.cuh"
+#include "group.cuh"
 #include "finalize.cuh"
 #include "a4.cuh"
 #include "../../include/rabung_census.h"
@@ -104,12 +105,19 @@ struct CZ_HANDLE {
     u32 n_small = 0;
     // device buffers
     Buf b_in, b_primes, b_profs, b_state, b_planes, b_summ, b_chunk, b_summp, b_didx, b_sidx,
-        b_slist, b_dlist, b_dpre, b_out, b_a4, b_counter, b_sreq, b_sout;
+        b_slist, b_dlist, b_dpre, b_out, b_a4, b_counter, b_sreq, b_sout,
+        b_groups, b_rgs, b_item0, b_jobs, b_lab, b_pw, b_gplanes, b_gplanes2;
     // host copies of the current plan
     std::vector<PrimeDesc> hp;
     std::vector<ProfDesc> hprof;
     std::vector<u32> h_chunk, h_summp, h_didx, h_sidx, h_slist, h_dlist;
+    std::vector<GroupDesc> hgroups;     // profiles filtered 32 per word (group.cuh)
+    std::vector<RowGroup> hrgs;
+    std::vector<u32> hitem0;
+    std::vector<uint2> hjobs;
     u32 n = 0, nprof = 0, ndense = 0, nsparse = 0, nchunks = 0, nsl = 0, ndl = 0;
+    u32 ntable = 0;                     // sparse primes with a profile outside the groups (table_kernel)
+    u32 lab_stride = 0, gmaxB = 0, lab_smem = 0;
     u32 table_smem = 0, dense_smem = 0;
     u32 flags = 0;
     bool have_plan = false;
@@ -179,6 +187,22 @@ bool build_static_tables(CZ_HANDLE *h) {
     return true;
 }
 
+// the primes below CHAIN_LIMIT, for counting table sizes on the host
+const std::vector<u32> &small_primes() {
+    static std::vector<u32> hs;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        std::vector<char> comp(CHAIN_LIMIT, 0);
+        for (u32 i = 2; i < CHAIN_LIMIT; ++i)
+            if (!comp[i]) {
+                hs.push_back(i);
+                if ((u64)i * i < CHAIN_LIMIT)
+                    for (u32 j = i * i; j < CHAIN_LIMIT; j += i) comp[j] = 1;
+            }
+    });
+    return hs;
+}
+
 u32 q_for(const cz_config &c, u32 r) { return c.q_cap[r] ? c.q_cap[r] : 16u; }
 
 // dense segment length in x (32 x steps), default DENSE_SEG
@@ -199,6 +223,166 @@ u32 qspec_for(const cz_config &c, pw_t p, u32 r, bool allow) {
 
 // host plan of one call
 constexpr u32 CZ_NOSPEC = 1u << 16;      // internal: plan without speculative thresholds
+constexpr u32 CZ_NOGROUP = 1u << 17;     // internal: every sparse profile on its own planes (serving)
+
+// Profiles below which a group is not worth forming: a group costs the same
+// whatever its members.
+constexpr u32 GROUP_MIN = 12;
+
+// compared planes and anchor stages of a group: least cost per visited anchor
+// and position of the row.  A stage costs F loads; beta is the bits it is worth
+// (-log2 of the chance that two colours agree in the compared planes); a step
+// of 32 anchors x 32 members leaves 1024 2^(-beta (t-1)) survivors, each
+// costing about seven loads' time in the queue and the screen.
+void group_plan(u32 r, u32 q, u32 &F, u32 &t) {
+    static const double beta2[10] = {0, 0, 1.0, 1.585, 2.0, 1.837, 1.848, 1.914, 2.0, 1.948};
+    static const double beta3[10] = {0, 0, 0, 0, 0, 2.322, 2.585, 2.807, 3.0, 2.880};
+    double bc = 0;
+    F = t = 0;
+    for (u32 f = r == 2 ? 1u : 2u; f <= (r == 2 ? 1u : r <= 4 ? 2u : 3u); ++f) {
+        const double beta = f == 3 ? beta3[r] : beta2[r];
+        const u32 lo = f == 1 ? G_TMIN1 : f == 2 ? G_TMIN2 : G_TMIN3, hi = f == 1 ? G_TMAX1 : f == 2 ? G_TMAX2 : G_TMAX3;
+        for (u32 k = lo; k <= hi && k <= q; ++k) {
+            const double c = (k * f + 1024.0 * std::exp2(-beta * (k - 1.0)) * 7.0) / (q - k + 1.0);
+            if (!t || c < bc) { F = f; t = k; bc = c; }
+        }
+    }
+}
+
+// elliptic cover with table radius at most B (group.cuh): E and the least D
+// with 3 E^2 D^2 >= 4 p^2, the largest row limit sqrt(E^2 + (H D / 2)^2) at most B
+bool cover_ellipse(u64 p, u32 B, u32 q, u32 &E, u32 &D) {
+    const long double H = q - 1.0L, k = 2.0L * p / std::sqrt(3.0L);
+    // E^2 + (H k / (2 E))^2 = (B - 4)^2, the larger root
+    const long double b2 = ((long double)B - 4.0L) * ((long double)B - 4.0L), disc = b2 * b2 - H * H * k * k;
+    if (B < 16u || disc <= 0) return false;
+    E = (u32)std::sqrt((b2 + std::sqrt(disc)) / 2.0L);
+    if (E < 16u) return false;
+    u64 d = (u64)(k / E);
+    auto ok = [&](u64 x) { return (unsigned __int128)3 * E * E * x * x >= (unsigned __int128)4 * p * p; };
+    while (d > 1 && ok(d - 1)) --d;
+    while (!ok(d)) ++d;
+    const u64 top = (u64)std::sqrt((long double)E * E + H * H * d * d / 4.0L) + 3u;
+    if (top > B || d >= p || E >= p || d > B_MAX || (q - 1u) * d > 2ull * B) return false;
+    D = (u32)d;
+    return true;
+}
+
+// the row whose limit is largest: E cos a + (H D / 2) sin a peaks at tan a = H D / (2 E)
+u32 group_apex(const GroupDesc &G) {
+    const double h = (G.q - 1.0) * G.D / 2.0;
+    return (u32)(G.D * h / std::sqrt(h * h + (double)G.E * G.E));
+}
+
+// row groups and items of one group; appended to rgs
+u32 group_items(GroupDesc &G, std::vector<RowGroup> &rgs) {
+    const u32 dn = std::min(group_narrow_end(G.t, G.F), (G.D / G_ROWS + 1u) * G_ROWS);
+    group_layout(G, dn);
+    G.rg0 = (u32)rgs.size();
+    u32 item = 0;
+    for (u32 d0 = 0; d0 <= G.D;) {
+        RowGroup R{};
+        R.item = item;
+        R.d0 = d0;
+        if (d0 < dn) {
+            R.nrows = std::min(G_ROWS, G.D + 1u - d0);
+            R.W = group_narrow_span(G.t, G.F, d0 + R.nrows - 1u);
+            u32 lim = 0;
+            for (u32 d = std::max(1u, d0); d < d0 + R.nrows; ++d) lim = std::max(lim, row_limit(G.E, G.D, G.B, G.q, d, 8u));
+            item += lim / 6u / R.W + 1u;
+        } else {
+            R.nrows = std::min(G_ROWS, G.D + 1u - d0);
+            const u32 wmax = group_wide_max(G.t, G.F), len = (d0 + R.nrows - 1u + 5u) / 6u;
+            R.ncol = (len + wmax - 1u) / wmax;
+            R.W = ((len + R.ncol - 1u) / R.ncol + 31u) & ~31u;
+            const u32 c0 = (((G.t - 1u) * d0 + 1u) >> 1) / 6u, sp = G.s * d0 / 6u;
+            const u32 lim = std::max(row_limit(G.E, G.D, G.B, G.q, d0, 8u),
+                                     row_limit(G.E, G.D, G.B, G.q, d0 + R.nrows - 1u, 8u));
+            const u32 apex = group_apex(G);             // the limit rises up to this row, then falls
+            const u32 top = apex >= d0 && apex < d0 + R.nrows ? G.B : lim;
+            const u32 bands = top / 6u >= c0 ? (top / 6u - c0) / sp + 1u : 0u;
+            item += bands * R.ncol;
+        }
+        rgs.push_back(R);
+        d0 += R.nrows;
+    }
+    G.nrg = (u32)rgs.size() - G.rg0;
+    return item;
+}
+
+// Profiles of one order whose primes lie within a factor 1.15 form groups of
+// up to 32 (the group runs its largest prime's cover, so nearer primes waste
+// less); the rest keep their own planes.  Sets ProfDesc.grouped and the
+// group's q as the members' speculative threshold.
+void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords, u64 &gwords2, u64 &pwwords) {
+    std::vector<u32> by[10];
+    for (u32 g = 0; g < h->nprof; ++g) {
+        const ProfDesc &D = h->hprof[g];
+        if (h->hp[D.prime].route == 2u && std::min(D.qspec, D.Q) >= 3u) by[D.r].push_back(g);
+    }
+    std::vector<u32> job_of(h->n, 0xFFFFFFFFu);
+    for (u32 r = 9; r >= 2; --r) {                   // costliest orders first: the launch ends on cheap items
+        auto &v = by[r];
+        std::stable_sort(v.begin(), v.end(), [h](u32 x, u32 y) {
+            return h->hp[h->hprof[x].prime].p > h->hp[h->hprof[y].prime].p;
+        });
+        for (size_t i = 0; i < v.size();) {
+            const pw_t pmax = h->hp[h->hprof[v[i]].prime].p;
+            size_t e = i;
+            u32 B = 0, q = 255;
+            pw_t pmin = pmax;
+            while (e < v.size() && e - i < 32) {
+                const ProfDesc &D = h->hprof[v[e]];
+                const PrimeDesc &P = h->hp[D.prime];
+                if ((u64)P.p + P.p / 7u < (u64)pmax) break;
+                B = std::max(B, P.B);
+                q = std::min(q, std::min(D.qspec, D.Q));
+                pmin = P.p;
+                ++e;
+            }
+            u32 Dd = 0;
+            u32 F = 0, t = 0;
+            group_plan(r, q, F, t);
+            u32 E = 0;
+            if (e - i < GROUP_MIN || !t || B >= pmin || !cover_ellipse(pmax, B, q, E, Dd) || Dd >= pmin) { ++i; continue; }
+            GroupDesc G{};
+            G.r = r; G.np = planes_for(r); G.F = F;
+            G.B = B; G.E = E; G.D = Dd; G.q = q; G.t = t; G.s = q - t + 1u;
+            G.n = (u32)(e - i);
+            G.nq = (u32)(std::upper_bound(primes_below.begin(), primes_below.end(), B) - primes_below.begin());
+            for (size_t k = i; k < e; ++k) {
+                ProfDesc &D = h->hprof[v[k]];
+                const pw_t p = h->hp[D.prime].p;
+                D.grouped = 1u;
+                D.qspec = q;
+                u32 &job = job_of[D.prime];
+                if (job == 0xFFFFFFFFu) { job = (u32)h->hjobs.size(); h->hjobs.push_back(make_uint2(D.prime, 0u)); }
+                h->hjobs[job].y = std::max(h->hjobs[job].y, G.nq);
+                G.prof[k - i] = v[k];
+                G.job[k - i] = job;
+                if ((u64)((p - 1u) >> 1) % r != 0u) G.sig |= 1u << (k - i);
+            }
+            h->hgroups.push_back(G);
+            i = e;
+        }
+    }
+    u32 items = 0, maxq = 0;
+    for (GroupDesc &G : h->hgroups) {
+        G.item0 = items;
+        h->hitem0.push_back(items);
+        items += group_items(G, h->hrgs);
+        G.off = gwords;
+        gwords += 6ull * G.CL * std::min(2u, G.np);  // CL is a multiple of 4: 16-byte aligned
+        G.off2 = gwords2;
+        gwords2 += 6ull * G.CL * (G.np > 2u ? G.np - 2u : 0u);
+        G.pwoff = pwwords;
+        pwwords += (u64)G.nq * G.np;
+        maxq = std::max(maxq, G.nq);
+        h->gmaxB = std::max(h->gmaxB, G.B);
+    }
+    h->hitem0.push_back(items);
+    h->lab_stride = (maxq + 63u) & ~63u;
+}
 
 int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
     const cz_config &c = h->cfg;
@@ -206,6 +390,8 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
     h->hprof.clear();
     h->h_didx.clear(); h->h_sidx.clear(); h->h_slist.clear(); h->h_dlist.clear();
     h->h_chunk.assign(1, 0u); h->h_summp.clear();
+    h->hgroups.clear(); h->hrgs.clear(); h->hitem0.clear(); h->hjobs.clear();
+    h->nsparse = 0; h->gmaxB = 0;
     u64 plane_words = 0;
     u32 max_slots_t = 8, max_slots_d = 8, max_nq = 0;
     u64 summ_slots = 0;
@@ -253,7 +439,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
             P.nwords = (2u * P.K0 + 8u + 3u) & ~3u;
             P.K2 = (B + 63u) / 64u + 4u;
             P.nwords2 = (2u * P.K2 + 8u + 3u) & ~3u;
-            h->h_sidx.push_back(i);
+            ++h->nsparse;
             max_slots_t = std::max(max_slots_t, hash_slots(P.m));
         } else {
             const u32 nh = (u32)((p - 1u) / 2u);           // < 2^32 for p < 2^33
@@ -284,11 +470,6 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
                 D.D = Ds[k];
                 D.qspec = qspec_for(c, p, r, !(flags & CZ_NOSPEC));
                 D.tpref = c.anchor_t[r] ? c.anchor_t[r] : anchor_pref(r, c.anchor_bits);
-                const u64 pw = ((u64)D.npp * (P.nwords + P.nwords2) + 7ull) & ~7ull;
-                D.plane_off = plane_words;              // multiple of 8 words: vector loads and tile copies align
-                plane_words += pw;
-                D.local = (u32)h->h_sidx.size() - 1u;
-                h->h_slist.push_back((u32)h->hprof.size());
             } else {
                 D.local = (u32)h->h_didx.size() - 1u;
                 h->h_dlist.push_back((u32)h->hprof.size());
@@ -300,8 +481,20 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
     h->n = n;
     h->nprof = (u32)h->hprof.size();
     h->ndense = (u32)h->h_didx.size();
-    h->nsparse = (u32)h->h_sidx.size();
     h->nchunks = h->h_chunk.back();
+    u64 gwords = 0, gwords2 = 0, pwwords = 0;
+    if (h->nsparse && !(flags & (CZ_NOSPEC | CZ_NOGROUP))) plan_groups(h, small_primes(), gwords, gwords2, pwwords);
+    for (u32 g = 0; g < h->nprof; ++g) {
+        ProfDesc &D = h->hprof[g];
+        const PrimeDesc &P = h->hp[D.prime];
+        if (P.route != 2u || D.grouped) continue;
+        D.plane_off = plane_words;                      // multiple of 8 words: vector loads and tile copies align
+        plane_words += ((u64)D.npp * (P.nwords + P.nwords2) + 7ull) & ~7ull;
+        if (h->h_sidx.empty() || h->h_sidx.back() != D.prime) h->h_sidx.push_back(D.prime);
+        D.local = (u32)h->h_sidx.size() - 1u;
+        h->h_slist.push_back(g);
+    }
+    h->ntable = (u32)h->h_sidx.size();
     // longest first: the persistent filter hands out profiles in list order,
     // so the costly ones (more stored planes, larger p) start first and the
     // launch ends on short profiles
@@ -315,22 +508,12 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
     // primes below the largest table end, for the table kernel's shared memory
     u32 maxB = 0;
     for (u32 i : h->h_sidx) maxB = std::max(maxB, h->hp[i].B);
-    if (h->nsparse) {
+    if (h->ntable) {
         const u32 nmax = 32u * ((maxB + 1u + 31u) / 32u + 1u);
-        // count primes below nmax on the host (static table is sorted)
-        static std::vector<u32> hs;
-        static std::once_flag once;
-        std::call_once(once, [] {
-            std::vector<char> comp(CHAIN_LIMIT, 0);
-            for (u32 i = 2; i < CHAIN_LIMIT; ++i)
-                if (!comp[i]) {
-                    hs.push_back(i);
-                    if ((u64)i * i < CHAIN_LIMIT)
-                        for (u32 j = i * i; j < CHAIN_LIMIT; j += i) comp[j] = 1;
-                }
-        });
+        const std::vector<u32> &hs = small_primes();
         max_nq = (u32)(std::lower_bound(hs.begin(), hs.end(), nmax) - hs.begin());
     }
+    h->lab_smem = max_slots_t * (u32)(sizeof(pw_t) + 2u) + 16u;
     h->table_smem = max_slots_t * (u32)(sizeof(pw_t) + 2u) + 8u + max_nq * 2u + 16u;
     if (h->table_smem > TABLE_DYN_SMEM) {
         h->err = "table shared memory above the per-block limit";
@@ -346,7 +529,15 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
         !ensure(h, h->b_chunk, 4ull * h->h_chunk.size()) ||
         !ensure(h, h->b_summp, 4ull * h->h_summp.size()) ||
         !ensure(h, h->b_didx, 4ull * h->ndense) ||
-        !ensure(h, h->b_sidx, 4ull * h->nsparse) ||
+        !ensure(h, h->b_sidx, 4ull * h->ntable) ||
+        !ensure(h, h->b_groups, sizeof(GroupDesc) * h->hgroups.size()) ||
+        !ensure(h, h->b_rgs, sizeof(RowGroup) * h->hrgs.size()) ||
+        !ensure(h, h->b_item0, 4ull * h->hitem0.size()) ||
+        !ensure(h, h->b_jobs, sizeof(uint2) * h->hjobs.size()) ||
+        !ensure(h, h->b_lab, 2ull * h->lab_stride * h->hjobs.size()) ||
+        !ensure(h, h->b_pw, 4ull * pwwords) ||
+        !ensure(h, h->b_gplanes, 4ull * gwords) ||
+        !ensure(h, h->b_gplanes2, 4ull * gwords2) ||
         !ensure(h, h->b_slist, 4ull * h->nsl) ||
         !ensure(h, h->b_dlist, 4ull * h->ndl) ||
         !ensure(h, h->b_dpre, 4ull * h->nprof) ||
@@ -362,7 +553,9 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
 int upload(CZ_HANDLE *h, cz_stats *s) {
     cudaStream_t st = h->st;
     size_t total = sizeof(PrimeDesc) * h->n + sizeof(ProfDesc) * h->nprof +
-                   4ull * (h->h_chunk.size() + h->h_summp.size() + h->ndense + h->nsparse + h->nsl + h->ndl) + 64 * 8;
+                   4ull * (h->h_chunk.size() + h->h_summp.size() + h->ndense + h->ntable + h->nsl + h->ndl) +
+                   sizeof(GroupDesc) * h->hgroups.size() + sizeof(RowGroup) * h->hrgs.size() +
+                   4ull * h->hitem0.size() + sizeof(uint2) * h->hjobs.size() + 64 * 12;
     if (h->pin_cap < total) {
         if (h->pin) cudaFreeHost(h->pin);
         h->pin = nullptr;
@@ -385,7 +578,11 @@ int upload(CZ_HANDLE *h, cz_stats *s) {
         !put(h->b_chunk, h->h_chunk.data(), 4ull * h->h_chunk.size()) ||
         !put(h->b_summp, h->h_summp.data(), 4ull * h->h_summp.size()) ||
         !put(h->b_didx, h->h_didx.data(), 4ull * h->ndense) ||
-        !put(h->b_sidx, h->h_sidx.data(), 4ull * h->nsparse) ||
+        !put(h->b_sidx, h->h_sidx.data(), 4ull * h->ntable) ||
+        !put(h->b_groups, h->hgroups.data(), sizeof(GroupDesc) * h->hgroups.size()) ||
+        !put(h->b_rgs, h->hrgs.data(), sizeof(RowGroup) * h->hrgs.size()) ||
+        !put(h->b_item0, h->hitem0.data(), 4ull * h->hitem0.size()) ||
+        !put(h->b_jobs, h->hjobs.data(), sizeof(uint2) * h->hjobs.size()) ||
         !put(h->b_slist, h->h_slist.data(), 4ull * h->nsl) ||
         !put(h->b_dlist, h->h_dlist.data(), 4ull * h->ndl))
         return CZ_ECUDA;
@@ -405,25 +602,73 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         ++launches;
     }
     rec(1);
-    if (h->nsparse) {
+    const u32 ngroups = (u32)h->hgroups.size();
+    if (ngroups) {
+        const u32 njobs = (u32)h->hjobs.size();
+        LabelArgs la;
+        la.primes = P<PrimeDesc>(h->b_primes);
+        la.state = P<ProfState>(h->b_state);
+        la.jobs = P<uint2>(h->b_jobs);
+        la.nchunk = std::max(2u, std::min(32u, 8u * (u32)h->sms / njobs));
+        la.lab = P<unsigned short>(h->b_lab);
+        la.stride = h->lab_stride;
+        la.small_primes = h->d_small;
+        plabel_kernel<<<njobs * la.nchunk, 256, h->lab_smem, st>>>(la);
+        GTableArgs ga;
+        ga.groups = P<GroupDesc>(h->b_groups);
+        ga.ngroups = ngroups;
+        ga.lab = la.lab;
+        ga.stride = la.stride;
+        ga.pw = P<u32>(h->b_pw);
+        ga.planes = P<u32>(h->b_gplanes);
+        ga.planes2 = P<u32>(h->b_gplanes2);
+        ga.chain = h->d_chain;
+        ga.small_primes = h->d_small;
+        const u32 qblk = h->lab_stride / 32u;
+        gpack_kernel<<<(ngroups * qblk + 7u) / 8u, 256, 0, st>>>(ga, qblk);
+        gtable_low_kernel<<<ngroups, 512, 0, st>>>(ga);
+        launches += 3;
+        for (u32 lo = G_LOW; lo <= h->gmaxB; lo *= 2u) {
+            const u32 nblk = (lo / 6u + 2u + 255u) / 256u;
+            gtable_level_kernel<<<ngroups * nblk, 256, 0, st>>>(ga, lo, nblk);
+            ++launches;
+        }
+    }
+    if (h->ntable) {
         TableArgs ta;
         ta.primes = P<PrimeDesc>(h->b_primes);
         ta.profs = P<ProfDesc>(h->b_profs);
         ta.state = P<ProfState>(h->b_state);
         ta.planes = P<u32>(h->b_planes);
         ta.sparse_primes = P<u32>(h->b_sidx);
-        ta.nsparse = h->nsparse;
+        ta.nsparse = h->ntable;
         ta.small_primes = h->d_small;
         ta.n_small = h->n_small;
         ta.chain = h->d_chain;
         ta.chain_limit = CHAIN_LIMIT;
-        const u32 grid = std::min<u32>(h->nsparse, (u32)h->sms);
+        const u32 grid = std::min<u32>(h->ntable, (u32)h->sms);
         table_kernel<<<grid, TABLE_THREADS, h->table_smem, st>>>(ta);
         ++launches;
     }
     rec(2);
+    if (h->nsl || ngroups) cudaMemsetAsync(h->b_counter.p, 0, 64, st);
+    if (ngroups) {
+        GFilterArgs fa;
+        fa.primes = P<PrimeDesc>(h->b_primes);
+        fa.profs = P<ProfDesc>(h->b_profs);
+        fa.state = P<ProfState>(h->b_state);
+        fa.groups = P<GroupDesc>(h->b_groups);
+        fa.item0 = P<u32>(h->b_item0);
+        fa.rgs = P<RowGroup>(h->b_rgs);
+        fa.ngroups = ngroups;
+        fa.nitems = h->hitem0.back();
+        fa.planes = P<u32>(h->b_gplanes);
+        fa.planes2 = P<u32>(h->b_gplanes2);
+        fa.next = P<u32>(h->b_counter) + 4;
+        gfilter_kernel<<<std::min(fa.nitems, (u32)h->sms), (G_WARPS + 2) * 32, G_SMEM, st>>>(fa);
+        ++launches;
+    }
     if (h->nsl) {
-        cudaMemsetAsync(h->b_counter.p, 0, 64, st);
         SparseArgs sa{};                       // serving fields stay null: one-call census
         sa.primes = P<PrimeDesc>(h->b_primes);
         sa.profs = P<ProfDesc>(h->b_profs);
@@ -533,7 +778,8 @@ void handle_close(CZ_HANDLE *h) {
     if (h->graph) cudaGraphDestroy(h->graph);
     Buf *bufs[] = {&h->b_in, &h->b_primes, &h->b_profs, &h->b_state, &h->b_planes, &h->b_summ, &h->b_chunk,
                    &h->b_summp, &h->b_didx, &h->b_sidx, &h->b_slist, &h->b_dlist, &h->b_dpre, &h->b_out,
-                   &h->b_a4, &h->b_counter, &h->b_sreq, &h->b_sout};
+                   &h->b_a4, &h->b_counter, &h->b_sreq, &h->b_sout, &h->b_groups, &h->b_rgs, &h->b_item0,
+                   &h->b_jobs, &h->b_lab, &h->b_pw, &h->b_gplanes, &h->b_gplanes2};
     for (Buf *b : bufs) if (b->p) cudaFree(b->p);
     if (h->pin) cudaFreeHost(h->pin);
     if (h->d_small) cudaFree(h->d_small);
@@ -569,6 +815,9 @@ int handle_open(const cz_config *cfg, CZ_HANDLE **out) {
     // goes to shared memory, two CTAs of TILE_WORDS words each per SM
     cudaFuncSetAttribute(sparse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TILE_WORDS * 4u));
     cudaFuncSetAttribute(sparse_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaFuncSetAttribute(gfilter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM);
+    cudaFuncSetAttribute(gfilter_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaFuncSetAttribute(plabel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
     if (!build_static_tables(h)) { handle_close(h); return CZ_ECUDA; }
     *out = h;
     return CZ_OK;

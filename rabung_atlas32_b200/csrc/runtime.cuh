@@ -353,7 +353,7 @@ void admit(cz_server *s) {
         }
         u32 mode = r->flags & CZ_AUTO;
         if (!mode) mode = CZ_AUTO;
-        int rc = plan(s->aux, r->primes.data(), n, mode);
+        int rc = plan(s->aux, r->primes.data(), n, mode | CZ_NOGROUP);
         if (rc) { finish(s, r, rc, s->aux->err); continue; }
         // the resident (sparse) part of the plan
         std::vector<PrimeDesc> hp;

@@ -110,14 +110,14 @@ table_kernel(TableArgs a) {
             TabProf t;
             t.r = D.r;
             t.magic = magic_of(D.r);
-            t.npp = D.npp;
+            t.npp = D.grouped ? 0u : D.npp;             // a grouped profile has no planes of its own
             t.sig = mod_small(P.sigma, D.r, t.magic);
             // a profile with a speculative threshold is certified by its best
             // run reaching q_spec (else it is re-run unspeculated, seed and
             // all), so its records never depend on the seed; the seed would
             // only raise its starting threshold when a stretch inside [1, B]
             // beat q_spec, which the margins make rare
-            t.seed = D.qspec == 0u ? 1u : 0u;
+            t.seed = D.qspec == 0u && !D.grouped ? 1u : 0u;
             t.base = a.planes + D.plane_off;
             t.odd = a.planes + D.plane_off + (u64)P.nwords * D.npp;
             tp[threadIdx.x] = t;
@@ -186,6 +186,7 @@ table_kernel(TableArgs a) {
             __syncwarp();
             for (u32 s = 0; s < nprof; ++s) {
                 const TabProf t = tp[s];
+                if (t.npp == 0u) continue;
                 TabWarp &W = tw[warp];
                 u32 prevw[4], stp[4], stn[4];
 #pragma unroll
