@@ -361,7 +361,7 @@ extern "C" int cz_census_dense_noalloc(const uint32_t *primes, uint32_t n, cz_pr
     ProfDesc *dD = reinterpret_cast<ProfDesc *>(base + L.profs);
     ProfState *dS = reinterpret_cast<ProfState *>(base + L.state);
     // setup_kernel re-initialises every ProfState this call uses
-    if (!launch(setup_kernel, dim3((n + 127) / 128), dim3(128), 0, st, dP, dD, dS, n)) return CZ_ECUDA;
+    if (!launch(setup_kernel, dim3((n + SETUP_WARPS - 1) / SETUP_WARPS), dim3(SETUP_WARPS * 32), 0, st, dP, dD, dS, n)) return CZ_ECUDA;
     u32 max_slots = 8;
     for (u32 i = 0; i < n; ++i) max_slots = std::max(max_slots, hash_slots(hp[i].m));
     DenseArgs da;
@@ -391,7 +391,7 @@ extern "C" int cz_census_dense_noalloc(const uint32_t *primes, uint32_t n, cz_pr
     if (!launch(dense_merge_kernel, dim3((nprof + 7) / 8), dim3(256), 0, st, ma, dl, nprof)) return CZ_ECUDA;
     OutRecord *dO = reinterpret_cast<OutRecord *>(base + L.out);
     const u32 *dpre = ma.prefix_out;
-    if (!launch(finalize_kernel, dim3((nprof + 127) / 128), dim3(128), 0, st, (const PrimeDesc *)dP,
+    if (!launch(finalize_kernel, dim3((nprof + FINAL_WARPS - 1) / FINAL_WARPS), dim3(FINAL_WARPS * 32), 0, st, (const PrimeDesc *)dP,
                 (const ProfDesc *)dD, (const ProfState *)dS, dpre, nprof, 0u, dO))
         return CZ_ECUDA;
     static_assert(sizeof(OutRecord) == sizeof(cz_profile), "record layout");

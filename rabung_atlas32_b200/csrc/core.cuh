@@ -597,7 +597,7 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
     auto rec = [&](int i) { if (timed) cudaEventRecord(h->ev[i], st); };
     rec(0);
     if (h->n) {
-        setup_kernel<<<(h->n + 127) / 128, 128, 0, st>>>(P<PrimeDesc>(h->b_primes), P<ProfDesc>(h->b_profs),
+        setup_kernel<<<(h->n + SETUP_WARPS - 1) / SETUP_WARPS, SETUP_WARPS * 32, 0, st>>>(P<PrimeDesc>(h->b_primes), P<ProfDesc>(h->b_profs),
                                                          P<ProfState>(h->b_state), h->n);
         ++launches;
     }
@@ -716,7 +716,7 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
     }
     rec(4);
     if (h->nprof) {
-        finalize_kernel<<<(h->nprof + 127) / 128, 128, 0, st>>>(
+        finalize_kernel<<<(h->nprof + FINAL_WARPS - 1) / FINAL_WARPS, FINAL_WARPS * 32, 0, st>>>(
             P<PrimeDesc>(h->b_primes), P<ProfDesc>(h->b_profs), P<ProfState>(h->b_state), P<u32>(h->b_dpre),
             h->nprof, (h->flags & CZ_VERIFY) ? 1u : 0u, P<OutRecord>(h->b_out));
         ++launches;

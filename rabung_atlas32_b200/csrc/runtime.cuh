@@ -424,7 +424,7 @@ void admit(cz_server *s) {
             table_smem = std::max(table_smem, s->aux->table_smem);
             cudaMemcpyAsync(s->d_primes + pb, hp.data(), sizeof(PrimeDesc) * np, cudaMemcpyHostToDevice, st);
             cudaMemcpyAsync(s->d_profs + gb, hg.data(), sizeof(ProfDesc) * ng, cudaMemcpyHostToDevice, st);
-            setup_kernel<<<(u32)((np + 127) / 128), 128, 0, st>>>(s->d_primes + pb, s->d_profs, s->d_state, (u32)np);
+            setup_kernel<<<(u32)((np + SETUP_WARPS - 1) / SETUP_WARPS), SETUP_WARPS * 32, 0, st>>>(s->d_primes + pb, s->d_profs, s->d_state, (u32)np);
             cudaMemsetAsync(s->d_a4err + sl, 0, 4, st);    // this request's A4 error word
             if (r->flags & CZ_A4)
                 a4_kernel<<<(u32)((np + A4_WARPS - 1) / A4_WARPS), A4_WARPS * 32, 0, st>>>(s->d_primes + pb, (u32)np,

@@ -743,7 +743,7 @@ __device__ __noinline__ void leave_profile(const SparseArgs &a, const ProfCtx &c
     const u32 left = atomicSub(&st->active, 1u) - 1u;
     const u32 claimed = (u32)*(volatile unsigned long long *)&st->claim;
     if (left != 0u || claimed < c.nitems || atomicCAS(&st->done, 0u, 1u) != 0u) return;
-    finalize_one(a.primes, a.profs, a.state, nullptr, g, a.verify, a.out);
+    finalize_one<false>(a.primes, a.profs, a.state, nullptr, g, a.verify, a.out, 0u);
     __threadfence();
     const u32 req = a.profs[g].req;
     if (atomicSub(&a.req_pending[req], 1u) == 1u) {
