@@ -99,6 +99,8 @@ struct CZ_HANDLE {
     int dev = 0;
     int sms = 148;
     cudaStream_t st = nullptr;
+    cudaStream_t st2 = nullptr;         // A4 counts beside the filter
+    cudaEvent_t fork = nullptr, join = nullptr;
     std::string err;
     u32 *d_small = nullptr;
     uint2 *d_chain = nullptr;
@@ -602,13 +604,28 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         ++launches;
     }
     rec(1);
-    const u32 ngroups = (u32)h->hgroups.size();
-    if (ngroups) {
-        const u32 njobs = (u32)h->hjobs.size();
+    // the A4 counts need the primes only and leave the GPU mostly idle (a long
+    // chain of curve operations per prime): they run beside the tables and the
+    // filter on a stream of their own, joined before the call's end
+    const bool a4 = (h->flags & CZ_A4) && h->n;
+    if (a4) {
+        cudaEventRecord(h->fork, st);
+        cudaStreamWaitEvent(h->st2, h->fork, 0);
+        if (timed) cudaEventRecord(h->ev[7], h->st2);
+        a4_kernel<<<(h->n + A4_WARPS - 1) / A4_WARPS, A4_WARPS * 32, 0, h->st2>>>(
+            P<PrimeDesc>(h->b_primes), h->n, P<u32>(h->b_a4), P<u32>(h->b_counter) + 8);
+        if (timed) cudaEventRecord(h->ev[8], h->st2);
+        cudaEventRecord(h->join, h->st2);
+        ++launches;
+    }
+    const u32 ngroups = (u32)h->hgroups.size(), njobs = (u32)h->hjobs.size();
+    if (njobs) {
         LabelArgs la;
         la.primes = P<PrimeDesc>(h->b_primes);
         la.state = P<ProfState>(h->b_state);
         la.jobs = P<uint2>(h->b_jobs);
+    // work counters and the A4 error word, before anything that runs beside
+    cudaMemsetAsync(h->b_counter.p, 0, 64, st);
         la.nchunk = std::max(2u, std::min(32u, 8u * (u32)h->sms / njobs));
         la.lab = P<unsigned short>(h->b_lab);
         la.stride = h->lab_stride;
@@ -651,7 +668,6 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         ++launches;
     }
     rec(2);
-    if (h->nsl || ngroups) cudaMemsetAsync(h->b_counter.p, 0, 64, st);
     if (ngroups) {
         GFilterArgs fa;
         fa.primes = P<PrimeDesc>(h->b_primes);
@@ -722,21 +738,15 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         ++launches;
     }
     rec(5);
-    if ((h->flags & CZ_A4) && h->n) {
-        // the A4 error word is cleared by every call that counts points, also
-        // when no sparse profile cleared the counter block above
-        cudaMemsetAsync(P<u32>(h->b_counter) + 8, 0, 4, st);
-        a4_kernel<<<(h->n + A4_WARPS - 1) / A4_WARPS, A4_WARPS * 32, 0, st>>>(P<PrimeDesc>(h->b_primes), h->n,
-                                                                           P<u32>(h->b_a4), P<u32>(h->b_counter) + 8);
-        ++launches;
-    }
+    if (a4) cudaStreamWaitEvent(st, h->join, 0);
     rec(6);
     return ck(h, cudaGetLastError(), "launch") ? CZ_OK : CZ_ECUDA;
 }
 
 void read_times(CZ_HANDLE *h, cz_stats *s) {
     float t[6] = {0};
-    for (int i = 0; i < 6; ++i) cudaEventElapsedTime(&t[i], h->ev[i], h->ev[i + 1]);
+    for (int i = 0; i < 5; ++i) cudaEventElapsedTime(&t[i], h->ev[i], h->ev[i + 1]);
+    if ((h->flags & CZ_A4) && h->n) cudaEventElapsedTime(&t[5], h->ev[7], h->ev[8]);
     s->ms_setup = t[0]; s->ms_table = t[1]; s->ms_sparse = t[2]; s->ms_dense = t[3];
     s->ms_finalize = t[4]; s->ms_a4 = t[5];
     cudaEventElapsedTime(&s->ms_device, h->ev[0], h->ev[6]);
@@ -804,10 +814,19 @@ int handle_open(const cz_config *cfg, CZ_HANDLE **out) {
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || h->dev < 0 || h->dev >= ndev) { delete h; return CZ_ECUDA; }
     cudaSetDevice(h->dev);
+    if (h->fork) cudaEventDestroy(h->fork);
+    if (h->join) cudaEventDestroy(h->join);
+    if (h->st2) cudaStreamDestroy(h->st2);
     cudaDeviceProp prop;
     cudaGetDeviceProperties(&prop, h->dev);
     h->sms = prop.multiProcessorCount;
-    if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess) { delete h; return CZ_ECUDA; }
+    if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&h->st2, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming) != cudaSuccess) {
+        handle_close(h);
+        return CZ_ECUDA;
+    }
     for (auto &e : h->ev) cudaEventCreate(&e);
     cudaFuncSetAttribute(table_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TABLE_DYN_SMEM);
     cudaFuncSetAttribute(dense_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
