@@ -197,6 +197,7 @@ struct PrimeDesc {
     u32 nprof;
     u32 route;       // 1 dense, 2 sparse
     u32 status;      // error bits set by kernels
+    u32 job;         // its row in the call's label matrix (group.cuh, table.cuh), if it has one
 };
 
 struct ProfDesc {

@@ -119,6 +119,7 @@ struct CZ_HANDLE {
     std::vector<uint2> hjobs;
     u32 n = 0, nprof = 0, ndense = 0, nsparse = 0, nchunks = 0, nsl = 0, ndl = 0;
     u32 ntable = 0;                     // sparse primes with a profile outside the groups (table_kernel)
+    bool tab_split = false;             // few of them: labels from the label matrix, several CTAs a prime
     u32 lab_stride = 0, gmaxB = 0, lab_smem = 0;
     u32 table_smem = 0, dense_smem = 0;
     u32 flags = 0;
@@ -312,6 +313,15 @@ u32 group_items(GroupDesc &G, std::vector<RowGroup> &rgs) {
     return item;
 }
 
+// row of prime i in the call's label matrix, at least nq labels long
+u32 need_labels(CZ_HANDLE *h, u32 i, u32 nq) {
+    PrimeDesc &P = h->hp[i];
+    if (P.job == 0xFFFFFFFFu) { P.job = (u32)h->hjobs.size(); h->hjobs.push_back(make_uint2(i, 0u)); }
+    h->hjobs[P.job].y = std::max(h->hjobs[P.job].y, nq);
+    h->lab_stride = std::max(h->lab_stride, (nq + 63u) & ~63u);     // rows hold whole 16-byte loads of labels
+    return P.job;
+}
+
 // Profiles of one order whose primes lie within a factor 1.15 form groups of
 // up to 32 (the group runs its largest prime's cover, so nearer primes waste
 // less); the rest keep their own planes.  Sets ProfDesc.grouped and the
@@ -322,7 +332,6 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
         const ProfDesc &D = h->hprof[g];
         if (h->hp[D.prime].route == 2u && std::min(D.qspec, D.Q) >= 3u) by[D.r].push_back(g);
     }
-    std::vector<u32> job_of(h->n, 0xFFFFFFFFu);
     for (u32 r = 9; r >= 2; --r) {                   // costliest orders first: the launch ends on cheap items
         auto &v = by[r];
         std::stable_sort(v.begin(), v.end(), [h](u32 x, u32 y) {
@@ -357,18 +366,15 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
                 const pw_t p = h->hp[D.prime].p;
                 D.grouped = 1u;
                 D.qspec = q;
-                u32 &job = job_of[D.prime];
-                if (job == 0xFFFFFFFFu) { job = (u32)h->hjobs.size(); h->hjobs.push_back(make_uint2(D.prime, 0u)); }
-                h->hjobs[job].y = std::max(h->hjobs[job].y, G.nq);
                 G.prof[k - i] = v[k];
-                G.job[k - i] = job;
+                G.job[k - i] = need_labels(h, D.prime, G.nq);
                 if ((u64)((p - 1u) >> 1) % r != 0u) G.sig |= 1u << (k - i);
             }
             h->hgroups.push_back(G);
             i = e;
         }
     }
-    u32 items = 0, maxq = 0;
+    u32 items = 0;
     for (GroupDesc &G : h->hgroups) {
         G.item0 = items;
         h->hitem0.push_back(items);
@@ -379,11 +385,9 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
         gwords2 += 6ull * G.CL * (G.np > 2u ? G.np - 2u : 0u);
         G.pwoff = pwwords;
         pwwords += (u64)G.nq * G.np;
-        maxq = std::max(maxq, G.nq);
         h->gmaxB = std::max(h->gmaxB, G.B);
     }
     h->hitem0.push_back(items);
-    h->lab_stride = (maxq + 63u) & ~63u;
 }
 
 int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
@@ -393,7 +397,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
     h->h_didx.clear(); h->h_sidx.clear(); h->h_slist.clear(); h->h_dlist.clear();
     h->h_chunk.assign(1, 0u); h->h_summp.clear();
     h->hgroups.clear(); h->hrgs.clear(); h->hitem0.clear(); h->hjobs.clear();
-    h->nsparse = 0; h->gmaxB = 0;
+    h->nsparse = 0; h->gmaxB = 0; h->lab_stride = 0;
     u64 plane_words = 0;
     u32 max_slots_t = 8, max_slots_d = 8, max_nq = 0;
     u64 summ_slots = 0;
@@ -409,6 +413,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
         P.first_prof = (u32)h->hprof.size();
         P.nprof = popc(P.mask);
         P.route = 0;
+        P.job = 0xFFFFFFFFu;
         if (!P.nprof) continue;
         bool sparse = false;
         if (mode == CZ_SPARSE) sparse = true;
@@ -497,6 +502,14 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
         h->h_slist.push_back(g);
     }
     h->ntable = (u32)h->h_sidx.size();
+    // few primes: their labels are computed over the whole GPU (table.cuh)
+    h->tab_split = h->ntable && 2u * h->ntable <= (u32)h->sms;
+    if (h->tab_split)
+        for (u32 i : h->h_sidx) {
+            const u32 nmax = 32u * ((h->hp[i].B + 1u + 31u) / 32u + 1u);
+            const std::vector<u32> &hs = small_primes();
+            need_labels(h, i, (u32)(std::lower_bound(hs.begin(), hs.end(), nmax) - hs.begin()));
+        }
     // longest first: the persistent filter hands out profiles in list order,
     // so the costly ones (more stored planes, larger p) start first and the
     // launch ends on short profiles
@@ -598,6 +611,8 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
     launches = 0;
     auto rec = [&](int i) { if (timed) cudaEventRecord(h->ev[i], st); };
     rec(0);
+    // work counters and the A4 error word, before anything that runs beside
+    cudaMemsetAsync(h->b_counter.p, 0, 64, st);
     if (h->n) {
         setup_kernel<<<(h->n + SETUP_WARPS - 1) / SETUP_WARPS, SETUP_WARPS * 32, 0, st>>>(P<PrimeDesc>(h->b_primes), P<ProfDesc>(h->b_profs),
                                                          P<ProfState>(h->b_state), h->n);
@@ -624,18 +639,19 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         la.primes = P<PrimeDesc>(h->b_primes);
         la.state = P<ProfState>(h->b_state);
         la.jobs = P<uint2>(h->b_jobs);
-    // work counters and the A4 error word, before anything that runs beside
-    cudaMemsetAsync(h->b_counter.p, 0, 64, st);
-        la.nchunk = std::max(2u, std::min(32u, 8u * (u32)h->sms / njobs));
+        la.nchunk = std::max(2u, std::min(96u, 8u * (u32)h->sms / njobs));
         la.lab = P<unsigned short>(h->b_lab);
         la.stride = h->lab_stride;
         la.small_primes = h->d_small;
         plabel_kernel<<<njobs * la.nchunk, 256, h->lab_smem, st>>>(la);
+        ++launches;
+    }
+    if (ngroups) {
         GTableArgs ga;
         ga.groups = P<GroupDesc>(h->b_groups);
         ga.ngroups = ngroups;
-        ga.lab = la.lab;
-        ga.stride = la.stride;
+        ga.lab = P<unsigned short>(h->b_lab);
+        ga.stride = h->lab_stride;
         ga.pw = P<u32>(h->b_pw);
         ga.planes = P<u32>(h->b_gplanes);
         ga.planes2 = P<u32>(h->b_gplanes2);
@@ -644,7 +660,7 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         const u32 qblk = h->lab_stride / 32u;
         gpack_kernel<<<(ngroups * qblk + 7u) / 8u, 256, 0, st>>>(ga, qblk);
         gtable_low_kernel<<<ngroups, 512, 0, st>>>(ga);
-        launches += 3;
+        launches += 2;
         for (u32 lo = G_LOW; lo <= h->gmaxB; lo *= 2u) {
             const u32 nblk = (lo / 6u + 2u + 255u) / 256u;
             gtable_level_kernel<<<ngroups * nblk, 256, 0, st>>>(ga, lo, nblk);
@@ -663,8 +679,11 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         ta.n_small = h->n_small;
         ta.chain = h->d_chain;
         ta.chain_limit = CHAIN_LIMIT;
-        const u32 grid = std::min<u32>(h->ntable, (u32)h->sms);
-        table_kernel<<<grid, TABLE_THREADS, h->table_smem, st>>>(ta);
+        ta.lab = h->tab_split ? P<unsigned short>(h->b_lab) : nullptr;
+        ta.lab_stride = h->lab_stride;
+        ta.nchunk = h->tab_split ? std::max(1u, std::min(64u, 2u * (u32)h->sms / h->ntable)) : 1u;
+        const u32 grid = ta.lab ? h->ntable * ta.nchunk : std::min<u32>(h->ntable, (u32)h->sms);
+        table_kernel<<<grid, TABLE_THREADS, ta.lab ? 0u : h->table_smem, st>>>(ta);
         ++launches;
     }
     rec(2);
@@ -795,6 +814,9 @@ void handle_close(CZ_HANDLE *h) {
     if (h->d_small) cudaFree(h->d_small);
     if (h->d_chain) cudaFree(h->d_chain);
     for (auto &e : h->ev) if (e) cudaEventDestroy(e);
+    if (h->fork) cudaEventDestroy(h->fork);
+    if (h->join) cudaEventDestroy(h->join);
+    if (h->st2) cudaStreamDestroy(h->st2);
     if (h->st) cudaStreamDestroy(h->st);
     delete h;
 }
@@ -814,9 +836,6 @@ int handle_open(const cz_config *cfg, CZ_HANDLE **out) {
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || h->dev < 0 || h->dev >= ndev) { delete h; return CZ_ECUDA; }
     cudaSetDevice(h->dev);
-    if (h->fork) cudaEventDestroy(h->fork);
-    if (h->join) cudaEventDestroy(h->join);
-    if (h->st2) cudaStreamDestroy(h->st2);
     cudaDeviceProp prop;
     cudaGetDeviceProperties(&prop, h->dev);
     h->sms = prop.multiProcessorCount;

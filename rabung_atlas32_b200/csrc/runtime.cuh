@@ -462,6 +462,9 @@ void admit(cz_server *s) {
         ta.n_small = s->h->n_small;
         ta.chain = s->h->d_chain;
         ta.chain_limit = CHAIN_LIMIT;
+        ta.lab = nullptr;
+        ta.lab_stride = 0;
+        ta.nchunk = 1;
         table_kernel<<<std::min<u32>(ta.nsparse, (u32)s->h->sms), TABLE_THREADS, table_smem, st>>>(ta);
         if (cudaStreamSynchronize(st) != cudaSuccess) {
             for (CzRequest *r : s->inflight) { release(s, r); finish(s, r, CZ_ECUDA, "set-up kernels failed"); }

@@ -34,6 +34,11 @@
 //    hence a certified lower bound on M (the role of the reference's
 //    seed_runs/finish_seed, small_table.cuh:64-136); a speculated profile is
 //    certified by its best run reaching the speculative threshold instead;
+//  * a CTA per prime takes 1.2 ms for one prime near 2^32, most of it the 4.8e4
+//    powers; calls with fewer primes than half the SMs compute those labels
+//    over the whole GPU first and split a prime's numerators over CTAs
+//    (measured: one prime 1.17 -> 0.04 ms; from about 74 primes on the split
+//    gains nothing: the CTAs fill the GPU either way);
 //  * the planes of one numerator step are stored with one instruction per
 //    word kind, lane b holding plane b.
 #pragma once
@@ -56,6 +61,11 @@ struct TableArgs {
     u32 n_small;
     const uint2 *chain;          // chain[n] = (index of q = spf(n) in small_primes | e << 24, n / q^e)
     u32 chain_limit;
+    // calls of few primes: labels of the small primes computed beforehand over
+    // the whole GPU (plabel_kernel, row PrimeDesc.job of lab_stride labels), and
+    // nchunk CTAs per prime, each a part of the numerators; nullptr, 1 otherwise
+    const unsigned short *lab;
+    u32 lab_stride, nchunk;
 };
 
 struct TabProf {            // per-profile constants of the CTA's prime
@@ -77,8 +87,9 @@ table_kernel(TableArgs a) {
     __shared__ unsigned short lab[TABLE_WARPS][TABLE_SUB + 1][32];
     __shared__ TabWarp tw[TABLE_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (u32 it = blockIdx.x; it < a.nsparse; it += gridDim.x) {
-        const u32 pi = a.sparse_primes[it];
+    for (u32 it = blockIdx.x; it < a.nsparse * a.nchunk; it += gridDim.x) {
+        const u32 chunk = it % a.nchunk;
+        const u32 pi = a.sparse_primes[it / a.nchunk];
         const PrimeDesc P = a.primes[pi];
         if (P.status & ST_ROOT) continue;   // not a prime, or no root of order m: the filter skips it
         const Mont M{P.p, P.ninv, P.one, P.r2};
@@ -87,8 +98,9 @@ table_kernel(TableArgs a) {
         // 4 u16 of padding, labels of the primes below the table end
         pw_t *keys = reinterpret_cast<pw_t *>(tsm);
         unsigned short *hl = reinterpret_cast<unsigned short *>(keys + slots);
-        unsigned short *plab = hl + slots + 4u;
-        build_root_hash(keys, hl, slots, M, P.z, P.m);
+        unsigned short *own = hl + slots + 4u;
+        const unsigned short *plab = a.lab ? a.lab + (size_t)P.job * a.lab_stride : own;
+        if (!a.lab) build_root_hash(keys, hl, slots, M, P.z, P.m);
         const u32 KS = (P.B + 1u + 31u) / 32u + 1u;            // steps: n in [0, 32*KS)
         const u32 nmax = 32u * KS;
         u32 lo = 0, hi = a.n_small;                              // primes below nmax
@@ -98,12 +110,13 @@ table_kernel(TableArgs a) {
         }
         const u32 nq = lo;
         u32 bad = (nmax > a.chain_limit) ? 1u : 0u;
-        for (u32 i = threadIdx.x; i < nq; i += blockDim.x) {
-            const pw_t y = mpow(to_mont((pw_t)a.small_primes[i], M), P.e, M);
-            u32 l = lookup_label(keys, hl, slots, y);
-            if (l == 0xFFFFu) { bad = 1; l = 0; }
-            plab[i] = (unsigned short)l;
-        }
+        if (!a.lab)
+            for (u32 i = threadIdx.x; i < nq; i += blockDim.x) {
+                const pw_t y = mpow(to_mont((pw_t)a.small_primes[i], M), P.e, M);
+                u32 l = lookup_label(keys, hl, slots, y);
+                if (l == 0xFFFFu) { bad = 1; l = 0; }
+                own[i] = (unsigned short)l;
+            }
         const u32 nprof = P.nprof;
         if (threadIdx.x < nprof) {
             const ProfDesc D = a.profs[P.first_prof + threadIdx.x];
@@ -130,7 +143,7 @@ table_kernel(TableArgs a) {
         if (lane < 8) tw[warp].cc[lane] = 0xFFFFFFFFu;
         const u32 K0 = P.K0, NW = P.nwords, K2 = P.K2, NW2 = P.nwords2;
         // guard words of both views (everything outside the written ranges)
-        for (u32 s = 0; s < nprof; ++s) {
+        for (u32 s = 0; s < nprof && chunk == 0u; ++s) {
             const TabProf t = tp[s];
             for (u32 w = threadIdx.x; w < NW; w += blockDim.x)
                 if (w + KS <= K0 || w >= K0 + KS)
@@ -141,9 +154,9 @@ table_kernel(TableArgs a) {
                     for (u32 k = 0; k < t.npp; ++k) t.odd[(size_t)w * t.npp + k] = 0u;
         }
         // warp chunk of steps [k0, k1), k0 even
-        u32 per = (KS + TABLE_WARPS - 1) / TABLE_WARPS;
+        u32 per = (KS + TABLE_WARPS * a.nchunk - 1) / (TABLE_WARPS * a.nchunk);
         per = (per + 1u) & ~1u;
-        const u32 k0 = min(KS, (u32)warp * per), k1 = min(KS, k0 + per);
+        const u32 k0 = min(KS, (chunk * TABLE_WARPS + (u32)warp) * per), k1 = min(KS, k0 + per);
         const u32 B = P.B;
         __syncwarp();
         for (u32 ks = k0; ks < k1; ks += TABLE_SUB) {
