@@ -124,6 +124,9 @@ struct CZ_HANDLE {
     u32 table_smem = 0, dense_smem = 0;
     u32 flags = 0;
     bool have_plan = false;
+    CZ_HANDLE *sub = nullptr;           // re-runs of missed speculations, on their own plan and buffers
+    bool sub_live = false;              // the last call re-ran profiles there (a replay repeats them)
+    bool borrowed = false;              // static tables belong to another handle
     cudaEvent_t ev[10]{};
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
@@ -216,11 +219,11 @@ u32 dense_seg(const cz_config &c) {
 
 // speculative threshold: floor(log_r p - margin_r), a low quantile of M for
 // random-looking colourings (M ~ log_r p); 0 disables
-u32 qspec_for(const cz_config &c, pw_t p, u32 r, bool allow) {
+u32 qspec_for(const cz_config &c, pw_t p, u32 r, bool allow, u32 level) {
     if (!allow || !c.speculate) return 0u;
     const double lg = std::log((double)p) / std::log((double)r);
     const double m = c.spec_margin10[r] / 10.0;
-    const double v = std::floor(lg - m);
+    const double v = std::floor(lg - m) - level;
     return v < 3.0 ? 0u : (u32)v;
 }
 
@@ -228,16 +231,20 @@ u32 qspec_for(const cz_config &c, pw_t p, u32 r, bool allow) {
 constexpr u32 CZ_NOSPEC = 1u << 16;      // internal: plan without speculative thresholds
 constexpr u32 CZ_NOGROUP = 1u << 17;     // internal: every sparse profile on its own planes (serving)
 
-// Profiles below which a group is not worth forming: a group costs the same
-// whatever its members.
-constexpr u32 GROUP_MIN = 12;
+// Cost of a profile on its own planes, in groups of its order and size (a group
+// costs the same whatever its members), and of a group besides its anchors, as
+// so much more p.  Measured on 40 windows of 61 primes: groups of near primes
+// of at least 1 / 4 / 8 / 12 members 42.4 / 41.7 / 45.8 / 53.4 ms, this cut with
+// a cost of 1/8, 1/5, 1/3 41.2 / 36.7 / 36.7 ms; 37 primes near 7e8 with 1/8,
+// 1/5, 1/3 2.49 / 2.47 / 2.07 ms on the device.
+constexpr double OWN_COST = 1.0 / 3.0, GROUP_FIXED = 2e7;
 
 // compared planes and anchor stages of a group: least cost per visited anchor
 // and position of the row.  A stage costs F loads; beta is the bits it is worth
 // (-log2 of the chance that two colours agree in the compared planes); a step
 // of 32 anchors x 32 members leaves 1024 2^(-beta (t-1)) survivors, each
 // costing about seven loads' time in the queue and the screen.
-void group_plan(u32 r, u32 q, u32 &F, u32 &t) {
+double group_plan(u32 r, u32 q, u32 &F, u32 &t) {
     static const double beta2[10] = {0, 0, 1.0, 1.585, 2.0, 1.837, 1.848, 1.914, 2.0, 1.948};
     static const double beta3[10] = {0, 0, 0, 0, 0, 2.322, 2.585, 2.807, 3.0, 2.880};
     double bc = 0;
@@ -250,25 +257,30 @@ void group_plan(u32 r, u32 q, u32 &F, u32 &t) {
             if (!t || c < bc) { F = f; t = k; bc = c; }
         }
     }
+    return bc;
 }
 
 // elliptic cover with table radius at most B (group.cuh): E and the least D
 // with 3 E^2 D^2 >= 4 p^2, the largest row limit sqrt(E^2 + (H D / 2)^2) at most B
 bool cover_ellipse(u64 p, u32 B, u32 q, u32 &E, u32 &D) {
     const long double H = q - 1.0L, k = 2.0L * p / std::sqrt(3.0L);
-    // E^2 + (H k / (2 E))^2 = (B - 4)^2, the larger root
-    const long double b2 = ((long double)B - 4.0L) * ((long double)B - 4.0L), disc = b2 * b2 - H * H * k * k;
-    if (B < 16u || disc <= 0) return false;
-    E = (u32)std::sqrt((b2 + std::sqrt(disc)) / 2.0L);
-    if (E < 16u) return false;
-    u64 d = (u64)(k / E);
-    auto ok = [&](u64 x) { return (unsigned __int128)3 * E * E * x * x >= (unsigned __int128)4 * p * p; };
-    while (d > 1 && ok(d - 1)) --d;
-    while (!ok(d)) ++d;
-    const u64 top = (u64)std::sqrt((long double)E * E + H * H * d * d / 4.0L) + 3u;
-    if (top > B || d >= p || E >= p || d > B_MAX || (q - 1u) * d > 2ull * B) return false;
-    D = (u32)d;
-    return true;
+    auto ok = [&](u64 d) { return (unsigned __int128)3 * E * E * d * d >= (unsigned __int128)4 * p * p; };
+    // E^2 + (H k / (2 E))^2 = (B - slack)^2, the larger root; D is rounded up,
+    // which moves the largest limit by up to about H / 2
+    for (u32 slack = 4; slack <= 4u + 2u * q && B > 16u + slack; slack += 4u) {
+        const long double b2 = ((long double)B - slack) * ((long double)B - slack), disc = b2 * b2 - H * H * k * k;
+        if (disc <= 0) return false;
+        E = (u32)std::sqrt((b2 + std::sqrt(disc)) / 2.0L);
+        u64 d = (u64)(k / E);
+        while (d > 1 && ok(d - 1)) --d;
+        while (!ok(d)) ++d;
+        const u64 top = (u64)std::sqrt((long double)E * E + H * H * d * d / 4.0L) + 3u;
+        if (top > B) continue;
+        if (d >= p || E >= p || d > B_MAX || (q - 1u) * d > 2ull * B) return false;
+        D = (u32)d;
+        return true;
+    }
+    return false;
 }
 
 // the row whose limit is largest: E cos a + (H D / 2) sin a peaks at tan a = H D / (2 E)
@@ -322,40 +334,63 @@ u32 need_labels(CZ_HANDLE *h, u32 i, u32 nq) {
     return P.job;
 }
 
-// Profiles of one order whose primes lie within a factor 1.15 form groups of
-// up to 32 (the group runs its largest prime's cover, so nearer primes waste
-// less); the rest keep their own planes.  Sets ProfDesc.grouped and the
-// group's q as the members' speculative threshold.
+// The sparse profiles of each order, in descending p, are cut into groups of up
+// to 32 and profiles kept on their own planes, at least modelled cost: a group
+// runs its largest prime's cover at its least threshold.  Cuts are considered
+// at 32 members and where p falls by more than 1/16 (a run of near primes is
+// best filled up).  Sets ProfDesc.grouped and the group's q as its members'
+// speculative threshold.
 void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords, u64 &gwords2, u64 &pwwords) {
     std::vector<u32> by[10];
     for (u32 g = 0; g < h->nprof; ++g) {
         const ProfDesc &D = h->hprof[g];
         if (h->hp[D.prime].route == 2u && std::min(D.qspec, D.Q) >= 3u) by[D.r].push_back(g);
     }
+    struct Cut { double cost; size_t from; u32 q; };
     for (u32 r = 9; r >= 2; --r) {                   // costliest orders first: the launch ends on cheap items
         auto &v = by[r];
-        std::stable_sort(v.begin(), v.end(), [h](u32 x, u32 y) {
-            return h->hp[h->hprof[x].prime].p > h->hp[h->hprof[y].prime].p;
-        });
-        for (size_t i = 0; i < v.size();) {
-            const pw_t pmax = h->hp[h->hprof[v[i]].prime].p;
-            size_t e = i;
-            u32 B = 0, q = 255;
-            pw_t pmin = pmax;
-            while (e < v.size() && e - i < 32) {
-                const ProfDesc &D = h->hprof[v[e]];
-                const PrimeDesc &P = h->hp[D.prime];
-                if ((u64)P.p + P.p / 7u < (u64)pmax) break;
-                B = std::max(B, P.B);
-                q = std::min(q, std::min(D.qspec, D.Q));
-                pmin = P.p;
-                ++e;
+        const size_t n = v.size();
+        if (!n) continue;
+        auto prime = [&](size_t k) { return h->hp[h->hprof[v[k]].prime].p; };
+        auto thr = [&](size_t k) { return std::min(h->hprof[v[k]].qspec, h->hprof[v[k]].Q); };
+        if (!std::is_sorted(v.begin(), v.end(), [h](u32 x, u32 y) {
+                return h->hp[h->hprof[x].prime].p > h->hp[h->hprof[y].prime].p; }))
+            std::stable_sort(v.begin(), v.end(), [h](u32 x, u32 y) {
+                return h->hp[h->hprof[x].prime].p > h->hp[h->hprof[y].prime].p;
+            });
+        double per[256];                             // modelled cost per position by q; 0: not asked yet
+        std::fill(per, per + 256, 0.0);
+        auto unit = [&](u32 q) {
+            u32 F, t;
+            if (per[q] == 0.0) per[q] = group_plan(r, q, F, t);
+            return per[q];
+        };
+        std::vector<Cut> best(n + 1, Cut{-1.0, 0, 0});
+        best[0].cost = 0;
+        for (size_t i = 0; i < n; ++i) {
+            if (best[i].cost < 0) continue;
+            const double pmax = (double)prime(i);
+            double own = 0;
+            u32 q = 255;
+            for (size_t e = i + 1; e <= n && e <= i + 32; ++e) {
+                const pw_t p = prime(e - 1);
+                q = std::min(q, thr(e - 1));
+                own += (double)p * unit(thr(e - 1)) * OWN_COST;
+                if (e < n && e < i + 32 && prime(e) >= p - p / 16u) continue;
+                const double group = (pmax + GROUP_FIXED) * unit(q);
+                const double c = best[i].cost + std::min(own, group);
+                if (best[e].cost < 0 || c < best[e].cost) best[e] = Cut{c, i, group <= own ? q : 0u};
             }
-            u32 Dd = 0;
-            u32 F = 0, t = 0;
+        }
+        for (size_t e = n; e > 0; e = best[e].from) {
+            const size_t i = best[e].from;
+            const u32 q = best[e].q;
+            if (!q) continue;
+            u32 F = 0, t = 0, E = 0, Dd = 0, B = 0;
             group_plan(r, q, F, t);
-            u32 E = 0;
-            if (e - i < GROUP_MIN || !t || B >= pmin || !cover_ellipse(pmax, B, q, E, Dd) || Dd >= pmin) { ++i; continue; }
+            for (size_t k = i; k < e; ++k) B = std::max(B, h->hp[h->hprof[v[k]].prime].B);
+            const pw_t pmin = prime(e - 1);
+            if (!t || B >= pmin || !cover_ellipse(prime(i), B, q, E, Dd) || Dd >= pmin) continue;
             GroupDesc G{};
             G.r = r; G.np = planes_for(r); G.F = F;
             G.B = B; G.E = E; G.D = Dd; G.q = q; G.t = t; G.s = q - t + 1u;
@@ -371,7 +406,6 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
                 if ((u64)((p - 1u) >> 1) % r != 0u) G.sig |= 1u << (k - i);
             }
             h->hgroups.push_back(G);
-            i = e;
         }
     }
     u32 items = 0;
@@ -390,7 +424,9 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
     h->hitem0.push_back(items);
 }
 
-int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
+// masks: the wanted orders of each prime (nullptr: every admissible one);
+// level: speculative thresholds lowered by so much (re-runs)
+int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = nullptr, u32 level = 0) {
     const cz_config &c = h->cfg;
     h->hp.assign(n, PrimeDesc{});
     h->hprof.clear();
@@ -407,7 +443,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
         if (p < 2u || (u64)p >= PW_LIMIT) { h->err = "prime out of domain: " + std::to_string(p); return CZ_EINVAL; }
         PrimeDesc &P = h->hp[i];
         P.p = p;
-        P.mask = p > 2u ? mask_of(p) : 0u;
+        P.mask = p > 2u ? mask_of(p) & (masks ? masks[i] : ~0u) : 0u;
         P.m = lcm_of_mask(P.mask);
         P.e = P.mask ? (p - 1u) / P.m : 0u;
         P.first_prof = (u32)h->hprof.size();
@@ -475,7 +511,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags) {
             if (sparse) {
                 D.Q = q_for(c, r);
                 D.D = Ds[k];
-                D.qspec = qspec_for(c, p, r, !(flags & CZ_NOSPEC));
+                D.qspec = qspec_for(c, p, r, !(flags & CZ_NOSPEC), level);
                 D.tpref = c.anchor_t[r] ? c.anchor_t[r] : anchor_pref(r, c.anchor_bits);
             } else {
                 D.local = (u32)h->h_didx.size() - 1u;
@@ -771,14 +807,16 @@ void read_times(CZ_HANDLE *h, cz_stats *s) {
     cudaEventElapsedTime(&s->ms_device, h->ev[0], h->ev[6]);
 }
 
+// status of every record: a speculative miss goes to *respec (profile index),
+// another status that the dense scan can settle to *fallback (prime index),
+// anything else refuses the call
 int check_records(CZ_HANDLE *h, std::vector<u32> *fallback, std::vector<u32> *respec = nullptr) {
     for (u32 g = 0; g < h->nprof; ++g) {
         const OutRecord &o = h->hout[g];
         if (o.status) {
             const PrimeDesc &P = h->hp[h->hprof[g].prime];
             if (respec && P.route == 2u && o.status == ST_SPEC) {
-                if (respec->empty() || respec->back() != h->hprof[g].prime)
-                    respec->push_back(h->hprof[g].prime);
+                respec->push_back(g);
                 continue;
             }
             if (fallback && P.route == 2u && !(o.status & (ST_ROOT | ST_LABEL | ST_VERIFY))) {
@@ -802,6 +840,7 @@ namespace {
 
 void handle_close(CZ_HANDLE *h) {
     if (!h) return;
+    handle_close(h->sub);
     cudaSetDevice(h->dev);
     if (h->gexec) cudaGraphExecDestroy(h->gexec);
     if (h->graph) cudaGraphDestroy(h->graph);
@@ -811,8 +850,8 @@ void handle_close(CZ_HANDLE *h) {
                    &h->b_jobs, &h->b_lab, &h->b_pw, &h->b_gplanes, &h->b_gplanes2};
     for (Buf *b : bufs) if (b->p) cudaFree(b->p);
     if (h->pin) cudaFreeHost(h->pin);
-    if (h->d_small) cudaFree(h->d_small);
-    if (h->d_chain) cudaFree(h->d_chain);
+    if (h->d_small && !h->borrowed) cudaFree(h->d_small);
+    if (h->d_chain && !h->borrowed) cudaFree(h->d_chain);
     for (auto &e : h->ev) if (e) cudaEventDestroy(e);
     if (h->fork) cudaEventDestroy(h->fork);
     if (h->join) cudaEventDestroy(h->join);
@@ -821,7 +860,8 @@ void handle_close(CZ_HANDLE *h) {
     delete h;
 }
 
-int handle_open(const cz_config *cfg, CZ_HANDLE **out) {
+// share: a handle on the same device whose static tables are used
+int handle_open(const cz_config *cfg, CZ_HANDLE **out, const CZ_HANDLE *share = nullptr) {
     if (!out) return CZ_EINVAL;
     *out = nullptr;
     CZ_HANDLE *h = new CZ_HANDLE();
@@ -856,7 +896,13 @@ int handle_open(const cz_config *cfg, CZ_HANDLE **out) {
     cudaFuncSetAttribute(gfilter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM);
     cudaFuncSetAttribute(gfilter_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     cudaFuncSetAttribute(plabel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    if (!build_static_tables(h)) { handle_close(h); return CZ_ECUDA; }
+    if (share) {
+        h->d_small = share->d_small; h->d_chain = share->d_chain; h->n_small = share->n_small;
+        h->borrowed = true;
+    } else if (!build_static_tables(h)) {
+        handle_close(h);
+        return CZ_ECUDA;
+    }
     *out = h;
     return CZ_OK;
 }
@@ -885,7 +931,8 @@ u64 plane_bytes(const cz_config &c, pw_t p, u32 flags) {
 }
 
 int census_impl(CZ_HANDLE *h, const pw_t *primes, uint32_t n, uint32_t flags, CZ_RECORD *out,
-                uint32_t out_cap, uint32_t *a4_out, cz_stats *stats, bool allow_fallback);
+                uint32_t out_cap, uint32_t *a4_out, cz_stats *stats, bool allow_fallback,
+                const u32 *masks = nullptr, u32 level = 0);
 
 // a batch whose plane pool would exceed the budget runs as consecutive waves
 int census_waves(CZ_HANDLE *h, const pw_t *primes, uint32_t n, uint32_t flags, CZ_RECORD *out,
@@ -926,7 +973,8 @@ int census_waves(CZ_HANDLE *h, const pw_t *primes, uint32_t n, uint32_t flags, C
 }
 
 int census_impl(CZ_HANDLE *h, const pw_t *primes, uint32_t n, uint32_t flags, CZ_RECORD *out,
-                       uint32_t out_cap, uint32_t *a4_out, cz_stats *stats, bool allow_fallback) {
+                       uint32_t out_cap, uint32_t *a4_out, cz_stats *stats, bool allow_fallback,
+                       const u32 *masks, u32 level) {
     if (!h) return CZ_EINVAL;
     cudaSetDevice(h->dev);
     h->err.clear();
@@ -934,10 +982,10 @@ int census_impl(CZ_HANDLE *h, const pw_t *primes, uint32_t n, uint32_t flags, CZ
     if (n == 0) { if (stats) *stats = s; return CZ_OK; }
     if (!primes || !out || ((flags & CZ_A4) && !a4_out)) { h->err = "null buffer"; return CZ_EINVAL; }
     if ((flags & CZ_AUTO) == 0) flags |= CZ_AUTO;
-    const u32 need = count_profiles(primes, n);
-    if (out_cap < need) { h->err = "output capacity below profile count"; return CZ_EINVAL; }
-    int rc = plan(h, primes, n, flags);
+    h->sub_live = false;
+    int rc = plan(h, primes, n, flags, masks, level);
     if (rc) return rc;
+    if (out_cap < h->nprof) { h->have_plan = false; h->err = "output capacity below profile count"; return CZ_EINVAL; }
     if (h->gexec) { cudaGraphExecDestroy(h->gexec); h->gexec = nullptr; }
     if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
     cudaEvent_t t0, t1;
@@ -988,44 +1036,59 @@ int census_impl(CZ_HANDLE *h, const pw_t *primes, uint32_t n, uint32_t flags, CZ
     }
     // the re-runs below re-plan the handle: take the primes and record slots first
     std::vector<pw_t> fb_p;
-    std::vector<u32> fb_first;
-    for (u32 pi : fb) { fb_p.push_back(h->hp[pi].p); fb_first.push_back(h->hp[pi].first_prof); }
+    std::vector<u32> fb_first, fb_mask;
+    for (u32 pi : fb) {
+        fb_p.push_back(h->hp[pi].p);
+        fb_first.push_back(h->hp[pi].first_prof);
+        fb_mask.push_back(h->hp[pi].mask);
+    }
     if (!rs.empty()) {
         // profiles whose best run stayed below the speculative threshold: the
-        // speculation was not certified, re-run those primes without it
-        std::vector<pw_t> sub;
-        for (u32 pi : rs) sub.push_back(h->hp[pi].p);
-        std::vector<u32> first(rs.size());
-        for (size_t k = 0; k < rs.size(); ++k) first[k] = h->hp[rs[k]].first_prof;
-        const u32 fflags = (flags & ~CZ_A4) | CZ_NOSPEC;
-        std::vector<CZ_RECORD> tmp(count_profiles(sub.data(), (u32)sub.size()));
-        cz_stats s2{};
-        rc = census_impl(h, sub.data(), (u32)sub.size(), fflags, tmp.data(), (u32)tmp.size(), nullptr, &s2, true);
-        if (rc) return rc;
-        u32 t = 0;
-        for (size_t k = 0; k < rs.size(); ++k) {
-            const u32 np = popc(mask_of(sub[k]));
-            for (u32 j = 0; j < np; ++j) out[first[k] + j] = tmp[t++];
+        // speculation was not certified.  Their orders alone are run again with
+        // the threshold one lower, and what misses that too without one, on a
+        // handle of their own, so this call's plan stays resident for a replay.
+        if (!h->sub && (rc = handle_open(&h->cfg, &h->sub, h))) { h->err = "re-run handle"; return rc; }
+        std::vector<pw_t> sp;
+        std::vector<u32> sm;
+        u32 last = 0xFFFFFFFFu;
+        for (u32 g : rs) {
+            const ProfDesc &D = h->hprof[g];
+            if (D.prime != last) { sp.push_back(h->hp[D.prime].p); sm.push_back(0u); }
+            last = D.prime;
+            sm.back() |= 1u << (D.r - 2u);
         }
-        s.n_respec = (u32)rs.size();
-        s.ms_respec = s2.ms_device;
-        h->have_plan = false;
+        u32 fflags = (flags & ~(CZ_AUTO | CZ_A4)) | CZ_SPARSE;
+        if (level) fflags |= CZ_NOSPEC;
+        std::vector<CZ_RECORD> tmp(rs.size());
+        cz_stats s2{};
+        rc = census_impl(h->sub, sp.data(), (u32)sp.size(), fflags, tmp.data(), (u32)tmp.size(), nullptr, &s2, true,
+                         sm.data(), level + 1u);
+        if (rc == CZ_EINVAL)                             // no filter for these orders alone
+            rc = census_impl(h->sub, sp.data(), (u32)sp.size(), (fflags & ~CZ_AUTO) | CZ_DENSE, tmp.data(),
+                             (u32)tmp.size(), nullptr, &s2, false, sm.data(), 0u);
+        if (rc) { h->err = h->sub->err; return rc; }
+        for (size_t k = 0; k < rs.size(); ++k) out[rs[k]] = tmp[k];
+        s.n_respec = (u32)sp.size();
+        s.n_fallback += s2.n_fallback;
+        s.ms_respec = s2.ms_device + s2.ms_respec;
+        s.kernels += s2.kernels;
+        h->sub_live = true;
+        h->have_plan = h->have_plan && h->sub->have_plan;
     }
     if (!fb.empty()) {
         // sparse primes whose seed could not certify a threshold: dense re-run
-        const std::vector<pw_t> &sub = fb_p;
-        const std::vector<u32> &first = fb_first;
         const u32 fflags = (flags & ~CZ_AUTO & ~CZ_A4) | CZ_DENSE;
-        std::vector<CZ_RECORD> tmp(count_profiles(sub.data(), (u32)sub.size()));
+        u32 np = 0;
+        for (u32 m : fb_mask) np += popc(m);
+        std::vector<CZ_RECORD> tmp(np);
         cz_stats s2{};
-        rc = census_impl(h, sub.data(), (u32)sub.size(), fflags, tmp.data(), (u32)tmp.size(), nullptr, &s2, false);
+        rc = census_impl(h, fb_p.data(), (u32)fb_p.size(), fflags, tmp.data(), np, nullptr, &s2, false,
+                         fb_mask.data());
         if (rc) return rc;
         u32 t = 0;
-        for (size_t k = 0; k < fb.size(); ++k) {
-            const u32 np = popc(mask_of(sub[k]));
-            for (u32 j = 0; j < np; ++j) out[first[k] + j] = tmp[t++];
-        }
-        s.n_fallback = (u32)fb.size();
+        for (size_t k = 0; k < fb_p.size(); ++k)
+            for (u32 j = 0; j < popc(fb_mask[k]); ++j) out[fb_first[k] + j] = tmp[t++];
+        s.n_fallback += (u32)fb.size();
         h->have_plan = false;   // the plan now describes the fallback batch
     }
     h->last = s;

@@ -23,7 +23,7 @@ def tup(recs):
 
 
 @pytest.mark.parametrize("lo,count", [(16384, 64), (70_001, 33), (1 << 20, 12), (1 << 20, 31), (1 << 20, 32),
-                                      (1 << 20, 97), (24_000_001, 65), (60_000_011, 40), (200_000_033, 24)])
+                                      (1 << 20, 97), (3_000_000, 33), (5_000_011, 31), (24_000_001, 65), (60_000_011, 40), (200_000_033, 24)])
 def test_groups_equal_dense(eng, lo, count):
     ps = sieve.primes_from(lo, count)
     assert tup(eng.profiles(ps, mode="sparse", a4=False)) == tup(eng.profiles(ps, mode="dense", a4=False))
