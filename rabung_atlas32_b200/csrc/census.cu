@@ -232,7 +232,7 @@ int cz_microbench(cz_handle *h, uint32_t kind, double *per_second) {
     for (int rep = 0; rep < 4; ++rep) {
         cudaEventRecord(h->ev[0], h->st);
         if (kind == 0) mb_alu_kernel<<<blocks, threads, 0, h->st>>>(iters, 0x9E3779B9u + rep, P<u32>(h->b_counter));
-        else mb_mont_kernel<<<blocks, threads, 0, h->st>>>(iters, p, M.ninv, P<u32>(h->b_counter));
+        else mb_mont_kernel<<<blocks, threads, 0, h->st>>>(iters, p, M.pinv, P<u32>(h->b_counter));
         cudaEventRecord(h->ev[1], h->st);
         if (!ck(h, cudaStreamSynchronize(h->st), "microbench")) return CZ_ECUDA;
         float ms = 0;

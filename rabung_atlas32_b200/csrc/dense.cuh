@@ -103,7 +103,7 @@ dense_scan_kernel(DenseArgs a) {
         __syncthreads();
         const u32 pi = cur_prime;
         const PrimeDesc P = a.primes[a.dense_idx[pi]];
-        const Mont M{P.p, P.ninv, P.one, P.r2};
+        const Mont M{P.p, P.pinv, P.one, P.r2};
         if (pi != prev_prime) {
             slots = hash_slots(P.m);
             labs = reinterpret_cast<unsigned short *>(keys + slots);

@@ -80,7 +80,7 @@ setup_kernel(PrimeDesc *primes, ProfDesc *profs, ProfState *state, u32 n) {
     if (!is_prime_warp(P.p, lane)) status |= ST_ROOT;
     if (P.p > 2u) {
         const Mont M = make_mont(P.p);
-        P.ninv = M.ninv; P.one = M.one; P.r2 = M.r2;
+        P.pinv = M.pinv; P.one = M.one; P.r2 = M.r2;
         P.z = M.one;
         if (P.m > 1u) {
             P.z = 0u;
@@ -169,7 +169,7 @@ __device__ inline void finalize_one(const PrimeDesc *primes, const ProfDesc *pro
     const PrimeDesc P = primes[D.prime];
     const unsigned long long best = *(const volatile unsigned long long *)&state[g].best;
     const u32 sstatus = *(const volatile u32 *)&state[g].status;
-    const Mont M{P.p, P.ninv, P.one, P.r2};
+    const Mont M{P.p, P.pinv, P.one, P.r2};
     const pw_t p = P.p, ex = (p - 1u) / D.r;
     const u32 r = D.r;
     u32 status = P.status | sstatus;

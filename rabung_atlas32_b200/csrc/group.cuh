@@ -257,7 +257,7 @@ plabel_kernel(LabelArgs a) {
     const u32 chunk = blockIdx.x % a.nchunk;
     const PrimeDesc P = a.primes[job.x];
     if (P.status & ST_ROOT) return;              // refused: its member is masked out of the filter
-    const Mont M{P.p, P.ninv, P.one, P.r2};
+    const Mont M{P.p, P.pinv, P.one, P.r2};
     const u32 slots = hash_slots(P.m);
     pw_t *keys = reinterpret_cast<pw_t *>(lsm);
     unsigned short *hl = reinterpret_cast<unsigned short *>(keys + slots);
@@ -632,7 +632,7 @@ __device__ __forceinline__ void gcomplete(const GShared &sh, const GroupDesc &G,
     const ProfDesc &D = a.profs[g];
     const PrimeDesc &Q = a.primes[D.prime];
     const pw_t p = Q.p;
-    const Mont M{p, Q.ninv, Q.one, Q.r2};
+    const Mont M{p, Q.pinv, Q.one, Q.r2};
     const u32 r = G.r;
     const pw_t dinv = mpow(to_mont((pw_t)d, M), p - 2u, M);
     const pw_t x = mmul((pw_t)b, dinv, M);

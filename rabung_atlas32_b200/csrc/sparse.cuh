@@ -802,7 +802,7 @@ __device__ __noinline__ void load_profile(const SparseArgs &a, u32 gprof, ProfCt
     ProfCtx c;
     c.p = PR.p; c.r = PD.r; c.np = PD.np; c.npp = PD.npp; c.Q = PD.Q; c.D = PD.D; c.B = PR.B;
     c.NW = PR.nwords; c.NW2 = PR.nwords2; c.OFF = 32u * PR.K0 + 31u; c.ex = (PR.p - 1u) / PD.r;
-    c.M = Mont{PR.p, PR.ninv, PR.one, PR.r2};
+    c.M = Mont{PR.p, PR.pinv, PR.one, PR.r2};
     c.P = a.planes + PD.plane_off;
     c.base = View{c.P, c.OFF, -(i32)PR.B, (i32)PR.B, 1u, 0u, 0u};
     // odd view: n = 2i + 1 in [-B, B]  <=>  i in [ceil((-B-1)/2), floor((B-1)/2)]

@@ -92,7 +92,7 @@ table_kernel(TableArgs a) {
         const u32 pi = a.sparse_primes[it / a.nchunk];
         const PrimeDesc P = a.primes[pi];
         if (P.status & ST_ROOT) continue;   // not a prime, or no root of order m: the filter skips it
-        const Mont M{P.p, P.ninv, P.one, P.r2};
+        const Mont M{P.p, P.pinv, P.one, P.r2};
         const u32 slots = hash_slots(P.m);
         // shared layout: root hash keys (slots words), their labels (slots u16),
         // 4 u16 of padding, labels of the primes below the table end
