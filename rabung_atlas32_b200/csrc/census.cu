@@ -383,6 +383,9 @@ extern "C" int cz_census_dense_noalloc(const uint32_t *primes, uint32_t n, cz_pr
     da.summ = reinterpret_cast<Summ *>(base + L.summ);
     da.state = dS;
     da.seg = DENSE_SEG;
+    da.chunk0 = 0;
+    da.lab_off = nullptr;                           // no scratch for labels: a power for every x
+    da.lab = nullptr;
     if (!launch(dense_scan_kernel, dim3(std::max(1u, std::min(chunk[nd], 1184u))), dim3(DENSE_WARPS * 32),
                 max_slots * 6u + 16u, st, da))
         return CZ_ECUDA;

@@ -108,11 +108,16 @@ struct CZ_HANDLE {
     // device buffers
     Buf b_in, b_primes, b_profs, b_state, b_planes, b_summ, b_chunk, b_summp, b_didx, b_sidx,
         b_slist, b_dlist, b_dpre, b_out, b_a4, b_counter, b_sreq, b_sout,
-        b_groups, b_rgs, b_item0, b_jobs, b_lab, b_pw, b_gplanes, b_gplanes2;
+        b_dlab, b_dlaboff, b_dlabp, b_groups, b_rgs, b_item0, b_jobs, b_lab, b_pw, b_gplanes, b_gplanes2;
     // host copies of the current plan
     std::vector<PrimeDesc> hp;
     std::vector<ProfDesc> hprof;
     std::vector<u32> h_chunk, h_summp, h_didx, h_sidx, h_slist, h_dlist;
+    // dense scan: waves of primes whose label arrays fit the pool together
+    struct DenseWave { u32 i0, i1, lchunk0, lchunks, chunk0, chunk1; };
+    std::vector<u64> h_dlaboff;         // per dense-local prime (NO_LABELS: powers in the scan)
+    std::vector<u32> h_dlabp;           // label chunks (prefix)
+    std::vector<DenseWave> hwaves;
     std::vector<GroupDesc> hgroups;     // profiles filtered 32 per word (group.cuh)
     std::vector<RowGroup> hrgs;
     std::vector<u32> hitem0;
@@ -225,6 +230,48 @@ u32 qspec_for(const cz_config &c, pw_t p, u32 r, bool allow, u32 level) {
     const double m = c.spec_margin10[r] / 10.0;
     const double v = std::floor(lg - m) - level;
     return v < 3.0 ? 0u : (u32)v;
+}
+
+// Dense primes from DENSE_LABEL_MIN_P on keep the labels of the x coprime to
+// 210 in memory (dense.cuh), in waves of at most DENSE_LABEL_WORDS 16-bit labels
+// (one prime below 2^33 takes 0.98e9 of them at most).  Where the line lies: 400
+// primes near 7e4 take 0.53 ms with the scan's own powers and 0.31 ms with kept
+// labels, 400 near 2e4 the same either way (0.39 ms).  Returns the pool's size
+// in labels.
+constexpr u64 DENSE_LABEL_MIN_P = 1u << 16, DENSE_LABEL_WORDS = 1ull << 31;
+u64 plan_dense_labels(CZ_HANDLE *h) {
+    h->h_dlaboff.clear();
+    h->h_dlabp.assign(1, 0u);
+    h->hwaves.clear();
+    if (!h->ndense) return 0;
+    CZ_HANDLE::DenseWave w{0, 0, 0, 0, 0, 0};
+    u64 used = 0, most = 0;
+    auto close = [&](u32 i) {
+        w.i1 = i;
+        w.chunk1 = h->h_chunk[i];
+        w.lchunks = h->h_dlabp[i] - w.lchunk0;
+        h->hwaves.push_back(w);
+        w = CZ_HANDLE::DenseWave{i, 0, h->h_dlabp[i], 0, h->h_chunk[i], 0};
+        most = std::max(most, used);
+        used = 0;
+    };
+    for (u32 i = 0; i < h->ndense; ++i) {
+        const pw_t p = h->hp[h->h_didx[i]].p;
+        u64 need = 0, off = NO_LABELS;
+        u32 nch = 0;
+        if (p >= DENSE_LABEL_MIN_P) {
+            const u32 nl = labels_below((u32)((p - 1u) / 2u));
+            need = ((u64)nl + DLABEL_HEAD + 7u) & ~7ull;
+            nch = (nl + DLABEL_CHUNK - 1u) / DLABEL_CHUNK;
+            if (used && used + need > DENSE_LABEL_WORDS) close(i);
+            off = used;
+            used += need;
+        }
+        h->h_dlaboff.push_back(off);
+        h->h_dlabp.push_back(h->h_dlabp.back() + nch);
+    }
+    close(h->ndense);
+    return most;
 }
 
 // host plan of one call
@@ -565,6 +612,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
         max_nq = (u32)(std::lower_bound(hs.begin(), hs.end(), nmax) - hs.begin());
     }
     h->lab_smem = max_slots_t * (u32)(sizeof(pw_t) + 2u) + 16u;
+    const u64 dlab = plan_dense_labels(h);
     h->table_smem = max_slots_t * (u32)(sizeof(pw_t) + 2u) + 8u + max_nq * 2u + 16u;
     if (h->table_smem > TABLE_DYN_SMEM) {
         h->err = "table shared memory above the per-block limit";
@@ -581,6 +629,9 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
         !ensure(h, h->b_summp, 4ull * h->h_summp.size()) ||
         !ensure(h, h->b_didx, 4ull * h->ndense) ||
         !ensure(h, h->b_sidx, 4ull * h->ntable) ||
+        !ensure(h, h->b_dlab, 2ull * dlab) ||
+        !ensure(h, h->b_dlaboff, 8ull * h->h_dlaboff.size()) ||
+        !ensure(h, h->b_dlabp, 4ull * h->h_dlabp.size()) ||
         !ensure(h, h->b_groups, sizeof(GroupDesc) * h->hgroups.size()) ||
         !ensure(h, h->b_rgs, sizeof(RowGroup) * h->hrgs.size()) ||
         !ensure(h, h->b_item0, 4ull * h->hitem0.size()) ||
@@ -606,7 +657,8 @@ int upload(CZ_HANDLE *h, cz_stats *s) {
     size_t total = sizeof(PrimeDesc) * h->n + sizeof(ProfDesc) * h->nprof +
                    4ull * (h->h_chunk.size() + h->h_summp.size() + h->ndense + h->ntable + h->nsl + h->ndl) +
                    sizeof(GroupDesc) * h->hgroups.size() + sizeof(RowGroup) * h->hrgs.size() +
-                   4ull * h->hitem0.size() + sizeof(uint2) * h->hjobs.size() + 64 * 12;
+                   4ull * h->hitem0.size() + sizeof(uint2) * h->hjobs.size() + 8ull * h->h_dlaboff.size() +
+                   4ull * h->h_dlabp.size() + 64 * 14;
     if (h->pin_cap < total) {
         if (h->pin) cudaFreeHost(h->pin);
         h->pin = nullptr;
@@ -630,6 +682,8 @@ int upload(CZ_HANDLE *h, cz_stats *s) {
         !put(h->b_summp, h->h_summp.data(), 4ull * h->h_summp.size()) ||
         !put(h->b_didx, h->h_didx.data(), 4ull * h->ndense) ||
         !put(h->b_sidx, h->h_sidx.data(), 4ull * h->ntable) ||
+        !put(h->b_dlaboff, h->h_dlaboff.data(), 8ull * h->h_dlaboff.size()) ||
+        !put(h->b_dlabp, h->h_dlabp.data(), 4ull * h->h_dlabp.size()) ||
         !put(h->b_groups, h->hgroups.data(), sizeof(GroupDesc) * h->hgroups.size()) ||
         !put(h->b_rgs, h->hrgs.data(), sizeof(RowGroup) * h->hrgs.size()) ||
         !put(h->b_item0, h->hitem0.data(), 4ull * h->hitem0.size()) ||
@@ -767,12 +821,32 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         da.chunk_prefix = P<u32>(h->b_chunk);
         da.summ_prefix = P<u32>(h->b_summp);
         da.nprimes = h->ndense;
-        da.nchunks = h->nchunks;
         da.summ = P<Summ>(h->b_summ);
         da.state = P<ProfState>(h->b_state);
         da.seg = dense_seg(h->cfg);
-        const u32 grid = std::min<u32>(h->nchunks, (u32)h->sms * 8u);
-        dense_scan_kernel<<<grid, DENSE_WARPS * 32, h->dense_smem, st>>>(da);
+        da.lab_off = P<u64>(h->b_dlaboff);
+        da.lab = P<unsigned short>(h->b_dlab);
+        for (const CZ_HANDLE::DenseWave &w : h->hwaves) {
+            if (w.lchunks) {
+                DLabelArgs dl;
+                dl.primes = da.primes;
+                dl.dense_idx = da.dense_idx;
+                dl.chunk_prefix = P<u32>(h->b_dlabp);
+                dl.i0 = w.i0;
+                dl.i1 = w.i1;
+                dl.chunk0 = w.lchunk0;
+                dl.lab_off = da.lab_off;
+                dl.lab = P<unsigned short>(h->b_dlab);
+                dl.state = da.state;
+                dlabel_kernel<<<w.lchunks, 256, h->dense_smem, st>>>(dl);
+                ++launches;
+            }
+            da.chunk0 = w.chunk0;
+            da.nchunks = w.chunk1;
+            const u32 grid = std::min<u32>(w.chunk1 - w.chunk0, (u32)h->sms * 8u);
+            dense_scan_kernel<<<grid, DENSE_WARPS * 32, h->dense_smem, st>>>(da);
+            ++launches;
+        }
         DenseMergeArgs ma;
         ma.primes = P<PrimeDesc>(h->b_primes);
         ma.profs = P<ProfDesc>(h->b_profs);
@@ -783,7 +857,7 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         ma.state = P<ProfState>(h->b_state);
         ma.prefix_out = P<u32>(h->b_dpre);
         dense_merge_kernel<<<(h->ndl + 7) / 8, 256, 0, st>>>(ma, P<u32>(h->b_dlist), h->ndl);
-        launches += 2;
+        ++launches;
     }
     rec(4);
     if (h->nprof) {
@@ -847,7 +921,7 @@ void handle_close(CZ_HANDLE *h) {
     Buf *bufs[] = {&h->b_in, &h->b_primes, &h->b_profs, &h->b_state, &h->b_planes, &h->b_summ, &h->b_chunk,
                    &h->b_summp, &h->b_didx, &h->b_sidx, &h->b_slist, &h->b_dlist, &h->b_dpre, &h->b_out,
                    &h->b_a4, &h->b_counter, &h->b_sreq, &h->b_sout, &h->b_groups, &h->b_rgs, &h->b_item0,
-                   &h->b_jobs, &h->b_lab, &h->b_pw, &h->b_gplanes, &h->b_gplanes2};
+                   &h->b_dlab, &h->b_dlaboff, &h->b_dlabp, &h->b_jobs, &h->b_lab, &h->b_pw, &h->b_gplanes, &h->b_gplanes2};
     for (Buf *b : bufs) if (b->p) cudaFree(b->p);
     if (h->pin) cudaFreeHost(h->pin);
     if (h->d_small && !h->borrowed) cudaFree(h->d_small);
@@ -889,6 +963,7 @@ int handle_open(const cz_config *cfg, CZ_HANDLE **out, const CZ_HANDLE *share = 
     for (auto &e : h->ev) cudaEventCreate(&e);
     cudaFuncSetAttribute(table_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TABLE_DYN_SMEM);
     cudaFuncSetAttribute(dense_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    cudaFuncSetAttribute(dlabel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
     // the filter stages its tiles in shared memory: the whole unified array
     // goes to shared memory, two CTAs of TILE_WORDS words each per SM
     cudaFuncSetAttribute(sparse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TILE_WORDS * 4u));

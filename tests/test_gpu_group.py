@@ -42,3 +42,14 @@ def test_composite_among_grouped_primes_is_refused(eng):
     with pytest.raises(CensusError, match="status"):
         eng.profiles(sieve.primes_from(1 << 25, 80) + [(1 << 25) + 1], mode="sparse", a4=True)
     assert time.perf_counter() - t0 < 5.0
+
+
+@pytest.mark.parametrize("lo,count", [(3, 60), (16 * 1024 - 300, 40), (65_536 - 120, 30), (1 << 17, 20), (9_999_991, 3)])
+def test_dense_scan_equals_oracle(eng, lo, count):
+    """The dense scan on both sides of the least prime whose labels are kept,
+    around one segment (8192 x) and one chunk, against the CPU oracle's walk."""
+    import oracle
+    ps = sieve.primes_from(lo, count)
+    for r in eng.profiles(ps, mode="dense", a4=False):
+        assert [(v.r, v.M, v.L, v.witness, v.K) for v in r.profiles] == \
+               [(v["r"], v["max"], v["prefix"], v["witness"], v["K"]) for v in oracle.profiles(r.p)], r.p
