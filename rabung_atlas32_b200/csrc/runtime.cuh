@@ -20,6 +20,11 @@
 //    and counts the request down; a request's last profile raises its done
 //    flag in mapped host memory, and the scheduler copies its records out
 //    while the kernel keeps running;
+//  * a request of up to about SRV_DIRECT_MS of filter time does not become
+//    resident: in the window it runs at once on the second handle, together with
+//    the others like it in one call, whose profiles form groups across requests
+//    (group.cuh; half the time of the per-profile filter and no bookkeeping per
+//    profile).  Only larger ones are worth a launch that yields;
 //  * primes routed to the dense scan (small p), primes whose sparse record
 //    needs the dense re-run, and requests larger than the whole plane arena
 //    (in waves of one slot's planes) are handled by a second handle in the
@@ -38,13 +43,13 @@ namespace {
 
 // census of `primes` into recs (and A4), on handle h
 int census_into(cz_handle *h, const std::vector<uint32_t> &primes, uint32_t flags, std::vector<cz_profile> &recs,
-                std::vector<uint32_t> &a4) {
+                std::vector<uint32_t> &a4, cz_stats *stats = nullptr) {
     const uint32_t n = (uint32_t)primes.size();
     recs.assign(cz_count_profiles(primes.data(), n), cz_profile{});
     a4.assign((flags & CZ_A4) ? n : 0u, 0u);
     if (n == 0) return CZ_OK;
     return cz_census(h, primes.data(), n, flags, recs.data(), (uint32_t)recs.size(),
-                     (flags & CZ_A4) ? a4.data() : nullptr, nullptr);
+                     (flags & CZ_A4) ? a4.data() : nullptr, stats);
 }
 
 // first-fit ranges of [0, cap)
@@ -79,6 +84,7 @@ struct CzRequest {
     uint64_t id = 0;
     uint32_t lo = 0, count = 0, flags = 0;
     bool given = false;                 // primes supplied by the caller
+    bool sieved = false;                // primes found by the device sieve
     int rc = -1;                        // -1 while pending
     std::string err;
     std::vector<uint32_t> primes;
@@ -103,6 +109,12 @@ constexpr u32 SRV_CAP_PRIMES = 1u << 20;       // resident primes
 constexpr u32 SRV_CAP_PROFILES = 1u << 22;     // resident profiles
 constexpr u32 SRV_CAP_SLOTS = 1u << 16;        // requests in flight
 constexpr int SRV_MIN_LAUNCH_US = 5000;        // a launch runs this long before it yields to arrivals
+// Requests of at most this much modelled filter time run directly in the
+// window, in calls of at most SRV_CALL_MS (what an arrival may have to wait for;
+// a prime near 2^32 takes about SRV_PRIME_MS, in proportion to p, in the groups
+// such calls form).  Measured on 24 requests of 1 to 256 primes submitted
+// together: all resident 46.5 ms, direct 25.8 ms.
+constexpr double SRV_DIRECT_MS = 20.0, SRV_CALL_MS = 40.0, SRV_PRIME_MS = 0.15;
 
 }  // namespace
 
@@ -303,6 +315,75 @@ void run_repairs(cz_server *s) {
     s->repair.clear();
 }
 
+double request_ms(const CzRequest *r) {
+    double t = 0;
+    for (u32 p : r->primes) t += (double)p;
+    return t * (SRV_PRIME_MS / 4294967296.0);
+}
+
+// requests run at once on the second handle, those of like flags together
+void run_direct(cz_server *s, std::vector<CzRequest *> &list) {
+    for (size_t i = 0; i < list.size();) {
+        std::vector<CzRequest *> call, rest;
+        std::vector<uint32_t> ps;
+        const uint32_t flags = list[i]->flags;
+        double ms = 0;
+        for (size_t k = i; k < list.size(); ++k) {
+            CzRequest *r = list[k];
+            const double t = request_ms(r);
+            if (r->flags != flags || (!call.empty() && ms + t > SRV_CALL_MS)) { rest.push_back(r); continue; }
+            ms += t;
+            call.push_back(r);
+            ps.insert(ps.end(), r->primes.begin(), r->primes.end());
+        }
+        std::copy(call.begin(), call.end(), list.begin() + i);
+        i += call.size();
+        std::copy(rest.begin(), rest.end(), list.begin() + i);
+        std::vector<cz_profile> recs;
+        std::vector<uint32_t> a4;
+        cz_stats st{};
+        int rc = census_into(s->aux, ps, flags | CZ_VERIFY, recs, a4, &st);
+        size_t g = 0, k = 0;
+        for (CzRequest *r : call) {
+            if (rc && call.size() > 1) {                   // one of them is refused: each by itself
+                const int own = census_into(s->aux, r->primes, flags | CZ_VERIFY, r->recs, r->a4, &st);
+                finish(s, r, own, own ? s->aux->err : std::string());
+                continue;
+            }
+            if (!rc) {
+                const size_t np = cz_count_profiles(r->primes.data(), (uint32_t)r->primes.size());
+                r->recs.assign(recs.begin() + g, recs.begin() + g + np);
+                g += np;
+                if (flags & CZ_A4) r->a4.assign(a4.begin() + k, a4.begin() + k + r->primes.size());
+                k += r->primes.size();
+            }
+            finish(s, r, rc, rc ? s->aux->err : std::string());
+        }
+        std::lock_guard<std::mutex> lk(s->m);
+        ++s->launches;
+        s->n_respec += st.n_respec;
+        s->n_fallback += st.n_fallback;
+    }
+}
+
+// primes of the requests that name an interval, by one call of the device sieve
+void sieve_requests(cz_server *s, const std::vector<CzRequest *> &batch) {
+    std::vector<uint32_t> lo, cnt;
+    std::vector<CzRequest *> rs;
+    uint64_t total = 0;
+    for (CzRequest *r : batch)
+        if (!r->given && !r->sieved) { rs.push_back(r); lo.push_back(r->lo); cnt.push_back(r->count); total += r->count; }
+    if (rs.empty() || total > (1ull << 28)) return;
+    std::vector<uint32_t> got(total), found(rs.size(), 0u);
+    if (cz_sieve(s->aux, lo.data(), cnt.data(), (uint32_t)rs.size(), got.data(), found.data())) return;
+    size_t off = 0;
+    for (size_t i = 0; i < rs.size(); ++i) {
+        rs[i]->primes.assign(got.begin() + off, got.begin() + off + found[i]);
+        rs[i]->sieved = true;
+        off += cnt[i];
+    }
+}
+
 // admit waiting requests while they fit; sieve, plan, upload, set up, table
 // and A4 on the whole GPU (no filter kernel runs now)
 void admit(cz_server *s) {
@@ -326,16 +407,18 @@ void admit(cz_server *s) {
         else
             back.push_back(r);
     };
+    std::vector<CzRequest *> direct;
+    sieve_requests(s, batch);
     for (size_t bi = 0; bi < batch.size(); ++bi) {
         CzRequest *r = batch[bi];
-        if (!back.empty()) { back.push_back(r); continue; }
-        if (!r->given) {
+        if (!r->given && !r->sieved) {                  // the joint sieve failed: each by itself
             std::vector<uint32_t> got(r->count);
             uint32_t found = 0;
             const int rc = cz_sieve(s->aux, &r->lo, &r->count, 1, got.data(), &found);
             if (rc) { finish(s, r, rc, cz_last_error(s->aux)); continue; }
             got.resize(found);
             r->primes.swap(got);
+            r->sieved = true;
         }
         const u32 n = (u32)r->primes.size();
         if (n == 0) { r->recs.clear(); r->a4.clear(); finish(s, r, CZ_OK); continue; }
@@ -351,6 +434,8 @@ void admit(cz_server *s) {
                 continue;
             }
         }
+        if ((r->flags & CZ_AUTO) != CZ_DENSE && request_ms(r) <= SRV_DIRECT_MS) { direct.push_back(r); continue; }
+        if (!back.empty()) { back.push_back(r); continue; }
         u32 mode = r->flags & CZ_AUTO;
         if (!mode) mode = CZ_AUTO;
         int rc = plan(s->aux, r->primes.data(), n, mode | CZ_NOGROUP);
@@ -471,6 +556,7 @@ void admit(cz_server *s) {
             s->inflight.clear();
         }
     }
+    run_direct(s, direct);
     s->blocked = !back.empty();
     if (!back.empty()) {
         std::lock_guard<std::mutex> lk(s->m);
