@@ -9,8 +9,12 @@ VDWA4V1 frames for an interval (docs/DATA_FORMAT.md).
 """
 from __future__ import annotations
 
+import array
 import ctypes
+import itertools
 from dataclasses import dataclass
+
+import numpy as np
 
 from . import _lib, codec
 
@@ -46,7 +50,13 @@ class Tuning:
 
 
 def _as_u32_array(values):
-    arr = (ctypes.c_uint32 * len(values))()
+    n = len(values)
+    if n:
+        try:                              # integers in range: converted in C
+            return (ctypes.c_uint32 * n).from_buffer(array.array("I", values))
+        except (TypeError, OverflowError):
+            pass
+    arr = (ctypes.c_uint32 * n)()
     for i, v in enumerate(values):
         if not 0 <= int(v) < 2 ** 32:
             raise ValueError(f"prime out of the 32-bit domain: {v}")
@@ -56,15 +66,14 @@ def _as_u32_array(values):
 
 def to_records(primes, out, a4v) -> list:
     """codec.Record list from C records grouped by prime in input order."""
-    recs, k = [], 0
-    for i, p in enumerate(primes):
-        rec = codec.Record(int(p), [], a4v[i] if a4v else 0)
-        for _ in range(bin(codec.expected_mask(p)).count("1") if p > 2 else 0):
-            v = out[k]
-            k += 1
-            rec.profiles.append(codec.Profile(v.r, v.M, v.L, v.witness, v.K))
-        recs.append(rec)
-    return recs
+    ps = np.array(primes, dtype=np.int64)
+    admissible = ((ps[:, None] - 1) % np.arange(2, 10) == 0).sum(axis=1) * (ps > 2)
+    ends = np.cumsum(admissible).tolist()
+    fields = np.frombuffer(out, dtype=out._type_)[:ends[-1] if ends else 0]
+    profiles = list(map(codec.Profile, *(fields[k].tolist() for k in ("r", "M", "L", "witness", "K"))))
+    starts = [0] + ends
+    return [codec.Record(p, profiles[a:b], v)
+            for p, a, b, v in zip(ps.tolist(), starts, ends, a4v or itertools.repeat(0))]
 
 
 def config(lib, device: int, t: Tuning) -> "_lib.cz_config":

@@ -224,9 +224,9 @@ u32 dense_seg(const cz_config &c) {
 
 // speculative threshold: floor(log_r p - margin_r), a low quantile of M for
 // random-looking colourings (M ~ log_r p); 0 disables
-u32 qspec_for(const cz_config &c, pw_t p, u32 r, bool allow, u32 level) {
+u32 qspec_for(const cz_config &c, double lg_p, u32 r, bool allow, u32 level) {
     if (!allow || !c.speculate) return 0u;
-    const double lg = std::log((double)p) / std::log((double)r);
+    const double lg = lg_p / std::log((double)r);
     const double m = c.spec_margin10[r] / 10.0;
     const double v = std::floor(lg - m) - level;
     return v < 3.0 ? 0u : (u32)v;
@@ -342,26 +342,26 @@ u32 group_items(GroupDesc &G, std::vector<RowGroup> &rgs) {
     group_layout(G, dn);
     G.rg0 = (u32)rgs.size();
     u32 item = 0;
+    const u32 apex = group_apex(G);                     // the limit rises up to this row, then falls
+    const u32 wmax = group_wide_max(G.t, G.F);
     for (u32 d0 = 0; d0 <= G.D;) {
         RowGroup R{};
         R.item = item;
         R.d0 = d0;
+        R.nrows = std::min(G_ROWS, G.D + 1u - d0);
+        if (d0 < dn) R.nrows = std::min(R.nrows, dn - d0);
+        const u32 d1 = d0 + R.nrows - 1u;
+        const u32 top = apex >= d0 && apex <= d1
+                            ? G.B
+                            : row_limit(G.E, G.D, G.B, G.q, apex < d0 ? std::max(1u, d0) : d1, 8u);
         if (d0 < dn) {
-            R.nrows = std::min(G_ROWS, G.D + 1u - d0);
-            R.W = group_narrow_span(G.t, G.F, d0 + R.nrows - 1u);
-            u32 lim = 0;
-            for (u32 d = std::max(1u, d0); d < d0 + R.nrows; ++d) lim = std::max(lim, row_limit(G.E, G.D, G.B, G.q, d, 8u));
-            item += lim / 6u / R.W + 1u;
+            R.W = group_narrow_span(G.t, G.F, d1);
+            item += top / 6u / R.W + 1u;
         } else {
-            R.nrows = std::min(G_ROWS, G.D + 1u - d0);
-            const u32 wmax = group_wide_max(G.t, G.F), len = (d0 + R.nrows - 1u + 5u) / 6u;
+            const u32 len = (d1 + 5u) / 6u;
             R.ncol = (len + wmax - 1u) / wmax;
             R.W = ((len + R.ncol - 1u) / R.ncol + 31u) & ~31u;
             const u32 c0 = (((G.t - 1u) * d0 + 1u) >> 1) / 6u, sp = G.s * d0 / 6u;
-            const u32 lim = std::max(row_limit(G.E, G.D, G.B, G.q, d0, 8u),
-                                     row_limit(G.E, G.D, G.B, G.q, d0 + R.nrows - 1u, 8u));
-            const u32 apex = group_apex(G);             // the limit rises up to this row, then falls
-            const u32 top = apex >= d0 && apex < d0 + R.nrows ? G.B : lim;
             const u32 bands = top / 6u >= c0 ? (top / 6u - c0) / sp + 1u : 0u;
             item += bands * R.ncol;
         }
@@ -429,15 +429,28 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
                 if (best[e].cost < 0 || c < best[e].cost) best[e] = Cut{c, i, group <= own ? q : 0u};
             }
         }
-        for (size_t e = n; e > 0; e = best[e].from) {
-            const size_t i = best[e].from;
+        std::vector<size_t> ends;                    // ends of the groups, largest primes first
+        for (size_t e = n; e > 0; e = best[e].from)
+            if (best[e].q) ends.push_back(e);
+        u32 B = 0, E = 0, Dd = 0, cq = 0, F = 0, t = 0;
+        pw_t cover_p = 0;                            // the prime the current cover was made for
+        for (size_t x = ends.size(); x-- > 0;) {
+            const size_t e = ends[x], i = best[e].from;
             const u32 q = best[e].q;
-            if (!q) continue;
-            u32 F = 0, t = 0, E = 0, Dd = 0, B = 0;
-            group_plan(r, q, F, t);
-            for (size_t k = i; k < e; ++k) B = std::max(B, h->hp[h->hprof[v[k]].prime].B);
-            const pw_t pmin = prime(e - 1);
-            if (!t || B >= pmin || !cover_ellipse(prime(i), B, q, E, Dd) || Dd >= pmin) continue;
+            const pw_t pmax = prime(i), pmin = prime(e - 1);
+            // a cover serves every smaller prime too: neighbouring groups share one,
+            // and with it their row groups, while that costs less than 1/1024
+            u32 own = 0;
+            for (size_t k = i; k < e; ++k) own = std::max(own, h->hp[h->hprof[v[k]].prime].B);
+            if (q != cq || own > B || (u64)pmax + pmax / 1024u < (u64)cover_p) {
+                cq = 0;
+                B = own;
+                group_plan(r, q, F, t);
+                if (!t || !cover_ellipse(pmax, B, q, E, Dd)) continue;
+                cq = q;
+                cover_p = pmax;
+            }
+            if (B >= pmin || Dd >= pmin) continue;
             GroupDesc G{};
             G.r = r; G.np = planes_for(r); G.F = F;
             G.B = B; G.E = E; G.D = Dd; G.q = q; G.t = t; G.s = q - t + 1u;
@@ -455,11 +468,18 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
             h->hgroups.push_back(G);
         }
     }
-    u32 items = 0;
+    u32 items = 0, own = 0;
+    const GroupDesc *pv = nullptr;
     for (GroupDesc &G : h->hgroups) {
         G.item0 = items;
         h->hitem0.push_back(items);
-        items += group_items(G, h->hrgs);
+        if (pv && pv->r == G.r && pv->B == G.B && pv->E == G.E && pv->D == G.D && pv->q == G.q) {
+            G.I0 = pv->I0; G.CL = pv->CL; G.rg0 = pv->rg0; G.nrg = pv->nrg;
+        } else {
+            own = group_items(G, h->hrgs);
+        }
+        pv = &G;
+        items += own;
         G.off = gwords;
         gwords += 6ull * G.CL * std::min(2u, G.np);  // CL is a multiple of 4: 16-byte aligned
         G.off2 = gwords2;
@@ -502,19 +522,10 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
         if (mode == CZ_SPARSE) sparse = true;
         else if (mode == CZ_AUTO) sparse = p >= c.sparse_min_p;
         u32 B = 0, Qmax = 0;
-        std::vector<u32> Ds;
         if (sparse) {
             for (u32 r = 2; r <= 9; ++r)
                 if (P.mask & (1u << (r - 2))) Qmax = std::max(Qmax, q_for(c, r));
             if (p < 4096u || Qmax + 1u >= p || !cover_B(p, Qmax, c.cover_n, B)) sparse = false;
-            if (sparse) {
-                for (u32 r = 2; r <= 9 && sparse; ++r) {
-                    if (!(P.mask & (1u << (r - 2)))) continue;
-                    u32 D = 0;
-                    if (!cover_D(p, B, q_for(c, r), D)) sparse = false;
-                    Ds.push_back(D);
-                }
-            }
             if (!sparse && mode == CZ_SPARSE) {
                 h->err = "sparse path unsupported for p = " + std::to_string(p);
                 return CZ_EINVAL;
@@ -546,7 +557,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
             h->h_chunk.push_back(h->h_chunk.back() + nch);
             max_slots_d = std::max(max_slots_d, hash_slots(P.m));
         }
-        u32 k = 0;
+        const double lg_p = sparse ? std::log((double)p) : 0.0;
         for (u32 r = 2; r <= 9; ++r) {
             if (!(P.mask & (1u << (r - 2)))) continue;
             ProfDesc D{};
@@ -557,15 +568,13 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
             D.out_slot = (u32)h->hprof.size();
             if (sparse) {
                 D.Q = q_for(c, r);
-                D.D = Ds[k];
-                D.qspec = qspec_for(c, p, r, !(flags & CZ_NOSPEC), level);
+                D.qspec = qspec_for(c, lg_p, r, !(flags & CZ_NOSPEC), level);
                 D.tpref = c.anchor_t[r] ? c.anchor_t[r] : anchor_pref(r, c.anchor_bits);
             } else {
                 D.local = (u32)h->h_didx.size() - 1u;
                 h->h_dlist.push_back((u32)h->hprof.size());
             }
             h->hprof.push_back(D);
-            ++k;
         }
     }
     h->n = n;
@@ -578,6 +587,8 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
         ProfDesc &D = h->hprof[g];
         const PrimeDesc &P = h->hp[D.prime];
         if (P.route != 2u || D.grouped) continue;
+        // with B from the largest cap a denominator bound exists for every order
+        if (!cover_D(P.p, P.B, D.Q, D.D)) { h->err = "no cover for p = " + std::to_string(P.p); return CZ_EINVAL; }
         D.plane_off = plane_words;                      // multiple of 8 words: vector loads and tile copies align
         plane_words += ((u64)D.npp * (P.nwords + P.nwords2) + 7ull) & ~7ull;
         if (h->h_sidx.empty() || h->h_sidx.back() != D.prime) h->h_sidx.push_back(D.prime);
