@@ -53,3 +53,12 @@ def test_dense_scan_equals_oracle(eng, lo, count):
     for r in eng.profiles(ps, mode="dense", a4=False):
         assert [(v.r, v.M, v.L, v.witness, v.K) for v in r.profiles] == \
                [(v["r"], v["max"], v["prefix"], v["witness"], v["K"]) for v in oracle.profiles(r.p)], r.p
+
+
+@pytest.mark.parametrize("lo,count", [(2, 400), (990, 12), (16_777_259, 33), (4_294_960_000, 40)])
+def test_a4_equals_oracle(eng, lo, count):
+    """Point counts on both sides of the direct count's limit (p = 1000), and
+    at odd batch sizes, against the CPU oracle."""
+    import oracle
+    ps = sieve.primes_from(lo, count)
+    assert eng.a4(ps) == [oracle.a4(p) if p > 2 else 0 for p in ps]
