@@ -206,15 +206,15 @@ int cz_a4(cz_handle *h, const uint32_t *primes, uint32_t n, uint32_t *a4_out) {
         hp[i] = PrimeDesc{};
         hp[i].p = primes[i];
     }
-    if (!ensure(h, h->b_primes, sizeof(PrimeDesc) * n) || !ensure(h, h->b_a4, 4ull * n) || !ensure(h, h->b_counter, 64))
+    if (!ensure(h, h->b_in, sizeof(PrimeDesc) * n) || !ensure(h, h->b_a4out, 4ull * n) || !ensure(h, h->b_count, 64))
         return CZ_ECUDA;
-    cudaMemcpyAsync(h->b_primes.p, hp.data(), sizeof(PrimeDesc) * n, cudaMemcpyHostToDevice, h->st);
-    cudaMemsetAsync(h->b_counter.p, 0, 64, h->st);
-    a4_kernel<<<(n + A4_WARPS - 1) / A4_WARPS, A4_WARPS * 32, 0, h->st>>>(P<PrimeDesc>(h->b_primes), n,
-                                                                      P<u32>(h->b_a4), P<u32>(h->b_counter) + 8);
-    cudaMemcpyAsync(a4_out, h->b_a4.p, 4ull * n, cudaMemcpyDeviceToHost, h->st);
+    cudaMemcpyAsync(h->b_in.p, hp.data(), sizeof(PrimeDesc) * n, cudaMemcpyHostToDevice, h->st);
+    cudaMemsetAsync(h->b_count.p, 0, 64, h->st);
+    a4_kernel<<<(n + A4_WARPS - 1) / A4_WARPS, A4_WARPS * 32, 0, h->st>>>(P<PrimeDesc>(h->b_in), n,
+                                                                      P<u32>(h->b_a4out), P<u32>(h->b_count) + 8);
+    cudaMemcpyAsync(a4_out, h->b_a4out.p, 4ull * n, cudaMemcpyDeviceToHost, h->st);
     u32 err = 0;
-    cudaMemcpyAsync(&err, P<u32>(h->b_counter) + 8, 4, cudaMemcpyDeviceToHost, h->st);
+    cudaMemcpyAsync(&err, P<u32>(h->b_count) + 8, 4, cudaMemcpyDeviceToHost, h->st);
     if (!ck(h, cudaStreamSynchronize(h->st), "a4")) return CZ_ECUDA;
     if (err) { h->err = "refused: A4 point count not certified"; return CZ_EREFUSED; }
     h->have_plan = false;
@@ -224,15 +224,15 @@ int cz_a4(cz_handle *h, const uint32_t *primes, uint32_t n, uint32_t *a4_out) {
 int cz_microbench(cz_handle *h, uint32_t kind, double *per_second) {
     if (!h || !per_second || kind > 1) return CZ_EINVAL;
     cudaSetDevice(h->dev);
-    if (!ensure(h, h->b_counter, 64)) return CZ_ECUDA;
+    if (!ensure(h, h->b_count, 64)) return CZ_ECUDA;
     const u32 blocks = (u32)h->sms * 8u, threads = 256, iters = kind == 0 ? 4096u : 1024u;
     const u32 p = 4294967291u;
     const Mont M = make_mont(p);
     float best = 1e30f;
     for (int rep = 0; rep < 4; ++rep) {
         cudaEventRecord(h->ev[0], h->st);
-        if (kind == 0) mb_alu_kernel<<<blocks, threads, 0, h->st>>>(iters, 0x9E3779B9u + rep, P<u32>(h->b_counter));
-        else mb_mont_kernel<<<blocks, threads, 0, h->st>>>(iters, p, M.pinv, P<u32>(h->b_counter));
+        if (kind == 0) mb_alu_kernel<<<blocks, threads, 0, h->st>>>(iters, 0x9E3779B9u + rep, P<u32>(h->b_count));
+        else mb_mont_kernel<<<blocks, threads, 0, h->st>>>(iters, p, M.pinv, P<u32>(h->b_count));
         cudaEventRecord(h->ev[1], h->st);
         if (!ck(h, cudaStreamSynchronize(h->st), "microbench")) return CZ_ECUDA;
         float ms = 0;

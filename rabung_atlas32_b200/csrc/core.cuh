@@ -105,9 +105,13 @@ struct CZ_HANDLE {
     u32 *d_small = nullptr;
     uint2 *d_chain = nullptr;
     u32 n_small = 0;
-    // device buffers
-    Buf b_in, b_primes, b_profs, b_state, b_planes, b_summ, b_chunk, b_summp, b_didx, b_sidx,
-        b_slist, b_dlist, b_dpre, b_out, b_a4, b_counter, b_sreq, b_sout,
+    // device memory of the current plan: descriptors and results in b_small (one
+    // copy in, one copy out), tables in b_big; the others below are places in them
+    Buf b_small, b_big;
+    size_t up_bytes = 0, down_off = 0, down_bytes = 0;
+    Buf b_in, b_count, b_a4out, b_sreq, b_sout;     // sieve, A4 and benchmark calls
+    Buf b_primes, b_profs, b_state, b_planes, b_summ, b_chunk, b_summp, b_didx, b_sidx,
+        b_slist, b_dlist, b_dpre, b_out, b_a4, b_counter,
         b_dlab, b_dlaboff, b_dlabp, b_groups, b_rgs, b_item0, b_jobs, b_lab, b_pw, b_gplanes, b_gplanes2;
     // host copies of the current plan
     std::vector<PrimeDesc> hp;
@@ -131,8 +135,8 @@ struct CZ_HANDLE {
     bool have_plan = false;
     CZ_HANDLE *sub = nullptr;           // re-runs of missed speculations, on their own plan and buffers
     bool sub_live = false;              // the last call re-ran profiles there (a replay repeats them)
-    bool borrowed = false;              // static tables belong to another handle
-    cudaEvent_t ev[10]{};
+    CZ_HANDLE *root = nullptr;          // a re-run handle's owner: its stream, events, pinned memory and tables are used
+    cudaEvent_t ev[12]{};
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     cz_stats last{};
@@ -491,6 +495,17 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
     h->hitem0.push_back(items);
 }
 
+// the host arrays of a plan that the device reads
+struct Part { Buf *at; const void *from; size_t bytes; };
+std::vector<Part> upload_parts(CZ_HANDLE *h) {
+    auto part = [](Buf &b, const auto &v) { return Part{&b, v.data(), sizeof(v[0]) * v.size()}; };
+    return {part(h->b_primes, h->hp), part(h->b_profs, h->hprof), part(h->b_chunk, h->h_chunk),
+            part(h->b_summp, h->h_summp), part(h->b_didx, h->h_didx), part(h->b_sidx, h->h_sidx),
+            part(h->b_dlaboff, h->h_dlaboff), part(h->b_dlabp, h->h_dlabp), part(h->b_groups, h->hgroups),
+            part(h->b_rgs, h->hrgs), part(h->b_item0, h->hitem0), part(h->b_jobs, h->hjobs),
+            part(h->b_slist, h->h_slist), part(h->b_dlist, h->h_dlist)};
+}
+
 // masks: the wanted orders of each prime (nullptr: every admissible one);
 // level: speculative thresholds lowered by so much (re-runs)
 int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = nullptr, u32 level = 0) {
@@ -630,79 +645,55 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
         return CZ_EINVAL;
     }
     h->dense_smem = max_slots_d * (u32)(sizeof(pw_t) + 2u) + 16u;
-    // device buffers
-    if (!ensure(h, h->b_primes, sizeof(PrimeDesc) * n) ||
-        !ensure(h, h->b_profs, sizeof(ProfDesc) * h->nprof) ||
-        !ensure(h, h->b_state, sizeof(ProfState) * h->nprof) ||
-        !ensure(h, h->b_planes, plane_words * 4ull) ||
-        !ensure(h, h->b_summ, sizeof(Summ) * summ_slots) ||
-        !ensure(h, h->b_chunk, 4ull * h->h_chunk.size()) ||
-        !ensure(h, h->b_summp, 4ull * h->h_summp.size()) ||
-        !ensure(h, h->b_didx, 4ull * h->ndense) ||
-        !ensure(h, h->b_sidx, 4ull * h->ntable) ||
-        !ensure(h, h->b_dlab, 2ull * dlab) ||
-        !ensure(h, h->b_dlaboff, 8ull * h->h_dlaboff.size()) ||
-        !ensure(h, h->b_dlabp, 4ull * h->h_dlabp.size()) ||
-        !ensure(h, h->b_groups, sizeof(GroupDesc) * h->hgroups.size()) ||
-        !ensure(h, h->b_rgs, sizeof(RowGroup) * h->hrgs.size()) ||
-        !ensure(h, h->b_item0, 4ull * h->hitem0.size()) ||
-        !ensure(h, h->b_jobs, sizeof(uint2) * h->hjobs.size()) ||
-        !ensure(h, h->b_lab, 2ull * h->lab_stride * h->hjobs.size()) ||
-        !ensure(h, h->b_pw, 4ull * pwwords) ||
-        !ensure(h, h->b_gplanes, 4ull * gwords) ||
-        !ensure(h, h->b_gplanes2, 4ull * gwords2) ||
-        !ensure(h, h->b_slist, 4ull * h->nsl) ||
-        !ensure(h, h->b_dlist, 4ull * h->ndl) ||
-        !ensure(h, h->b_dpre, 4ull * h->nprof) ||
-        !ensure(h, h->b_out, sizeof(OutRecord) * h->nprof) ||
-        !ensure(h, h->b_a4, 4ull * n) ||
-        !ensure(h, h->b_counter, 64))
-        return CZ_ECUDA;
+    // device memory: uploaded descriptors, then the results (counters, records,
+    // A4, states) that come back in one copy, in one buffer; tables in another
+    size_t small = 0, big = 0;
+    std::vector<std::pair<Buf *, size_t>> at_small, at_big;
+    auto place = [](std::vector<std::pair<Buf *, size_t>> &v, size_t &end, Buf &b, size_t bytes) {
+        v.push_back({&b, end});
+        end += (bytes + 255) & ~size_t(255);
+    };
+    for (const Part &x : upload_parts(h)) place(at_small, small, *x.at, x.bytes);
+    h->up_bytes = h->down_off = small;
+    place(at_small, small, h->b_counter, 64);
+    place(at_small, small, h->b_out, sizeof(OutRecord) * h->nprof);
+    place(at_small, small, h->b_a4, 4ull * n);
+    place(at_small, small, h->b_state, sizeof(ProfState) * h->nprof);
+    h->down_bytes = small - h->down_off;
+    place(at_small, small, h->b_dpre, 4ull * h->nprof);
+    place(at_big, big, h->b_planes, plane_words * 4ull);
+    place(at_big, big, h->b_summ, sizeof(Summ) * summ_slots);
+    place(at_big, big, h->b_dlab, 2ull * dlab);
+    place(at_big, big, h->b_lab, 2ull * h->lab_stride * h->hjobs.size());
+    place(at_big, big, h->b_pw, 4ull * pwwords);
+    place(at_big, big, h->b_gplanes, 4ull * gwords);
+    place(at_big, big, h->b_gplanes2, 4ull * gwords2);
+    h->have_plan = false;
+    if (!ensure(h, h->b_small, small) || !ensure(h, h->b_big, big)) return CZ_ECUDA;
+    for (auto &x : at_small) x.first->p = static_cast<char *>(h->b_small.p) + x.second;
+    for (auto &x : at_big) x.first->p = static_cast<char *>(h->b_big.p) + x.second;
     h->flags = flags;
     h->have_plan = true;
     return CZ_OK;
 }
 
 int upload(CZ_HANDLE *h, cz_stats *s) {
-    cudaStream_t st = h->st;
-    size_t total = sizeof(PrimeDesc) * h->n + sizeof(ProfDesc) * h->nprof +
-                   4ull * (h->h_chunk.size() + h->h_summp.size() + h->ndense + h->ntable + h->nsl + h->ndl) +
-                   sizeof(GroupDesc) * h->hgroups.size() + sizeof(RowGroup) * h->hrgs.size() +
-                   4ull * h->hitem0.size() + sizeof(uint2) * h->hjobs.size() + 8ull * h->h_dlaboff.size() +
-                   4ull * h->h_dlabp.size() + 64 * 14;
-    if (h->pin_cap < total) {
-        if (h->pin) cudaFreeHost(h->pin);
-        h->pin = nullptr;
-        h->pin_cap = 0;
-        if (!ck(h, cudaHostAlloc(&h->pin, total + total / 4, cudaHostAllocDefault), "cudaHostAlloc")) return CZ_ECUDA;
-        h->pin_cap = total + total / 4;
+    CZ_HANDLE *o = h->root ? h->root : h;               // owner of the pinned memory
+    const size_t total = std::max(h->up_bytes, h->down_bytes);
+    if (o->pin_cap < total) {
+        if (o->pin) cudaFreeHost(o->pin);
+        o->pin = nullptr;
+        o->pin_cap = 0;
+        if (!ck(h, cudaHostAlloc(&o->pin, total + total / 4, cudaHostAllocDefault), "cudaHostAlloc")) return CZ_ECUDA;
+        o->pin_cap = total + total / 4;
     }
-    // the host plan is staged in pinned memory and copied asynchronously
-    char *stage = static_cast<char *>(h->pin);
-    size_t bytes = 0;
-    auto put = [&](Buf &b, const void *src, size_t n) {
-        if (n == 0) return true;
-        std::memcpy(stage + bytes, src, n);
-        const bool ok = ck(h, cudaMemcpyAsync(b.p, stage + bytes, n, cudaMemcpyHostToDevice, st), "h2d");
-        bytes += (n + 63) & ~size_t(63);
-        return ok;
-    };
-    if (!put(h->b_primes, h->hp.data(), sizeof(PrimeDesc) * h->n) ||
-        !put(h->b_profs, h->hprof.data(), sizeof(ProfDesc) * h->nprof) ||
-        !put(h->b_chunk, h->h_chunk.data(), 4ull * h->h_chunk.size()) ||
-        !put(h->b_summp, h->h_summp.data(), 4ull * h->h_summp.size()) ||
-        !put(h->b_didx, h->h_didx.data(), 4ull * h->ndense) ||
-        !put(h->b_sidx, h->h_sidx.data(), 4ull * h->ntable) ||
-        !put(h->b_dlaboff, h->h_dlaboff.data(), 8ull * h->h_dlaboff.size()) ||
-        !put(h->b_dlabp, h->h_dlabp.data(), 4ull * h->h_dlabp.size()) ||
-        !put(h->b_groups, h->hgroups.data(), sizeof(GroupDesc) * h->hgroups.size()) ||
-        !put(h->b_rgs, h->hrgs.data(), sizeof(RowGroup) * h->hrgs.size()) ||
-        !put(h->b_item0, h->hitem0.data(), 4ull * h->hitem0.size()) ||
-        !put(h->b_jobs, h->hjobs.data(), sizeof(uint2) * h->hjobs.size()) ||
-        !put(h->b_slist, h->h_slist.data(), 4ull * h->nsl) ||
-        !put(h->b_dlist, h->h_dlist.data(), 4ull * h->ndl))
-        return CZ_ECUDA;
-    if (s) s->h2d_bytes = bytes;
+    // the host plan, laid out as on the device, in one copy
+    char *stage = static_cast<char *>(o->pin);
+    const char *base = static_cast<const char *>(h->b_small.p);
+    for (const Part &x : upload_parts(h))
+        if (x.bytes) std::memcpy(stage + (static_cast<const char *>(x.at->p) - base), x.from, x.bytes);
+    if (!ck(h, cudaMemcpyAsync(h->b_small.p, stage, h->up_bytes, cudaMemcpyHostToDevice, h->st), "h2d")) return CZ_ECUDA;
+    if (s) s->h2d_bytes = h->up_bytes;
     return CZ_OK;
 }
 
@@ -929,24 +920,36 @@ void handle_close(CZ_HANDLE *h) {
     cudaSetDevice(h->dev);
     if (h->gexec) cudaGraphExecDestroy(h->gexec);
     if (h->graph) cudaGraphDestroy(h->graph);
-    Buf *bufs[] = {&h->b_in, &h->b_primes, &h->b_profs, &h->b_state, &h->b_planes, &h->b_summ, &h->b_chunk,
-                   &h->b_summp, &h->b_didx, &h->b_sidx, &h->b_slist, &h->b_dlist, &h->b_dpre, &h->b_out,
-                   &h->b_a4, &h->b_counter, &h->b_sreq, &h->b_sout, &h->b_groups, &h->b_rgs, &h->b_item0,
-                   &h->b_dlab, &h->b_dlaboff, &h->b_dlabp, &h->b_jobs, &h->b_lab, &h->b_pw, &h->b_gplanes, &h->b_gplanes2};
+    Buf *bufs[] = {&h->b_small, &h->b_big, &h->b_in, &h->b_count, &h->b_a4out, &h->b_sreq, &h->b_sout};
     for (Buf *b : bufs) if (b->p) cudaFree(b->p);
-    if (h->pin) cudaFreeHost(h->pin);
-    if (h->d_small && !h->borrowed) cudaFree(h->d_small);
-    if (h->d_chain && !h->borrowed) cudaFree(h->d_chain);
-    for (auto &e : h->ev) if (e) cudaEventDestroy(e);
-    if (h->fork) cudaEventDestroy(h->fork);
-    if (h->join) cudaEventDestroy(h->join);
-    if (h->st2) cudaStreamDestroy(h->st2);
-    if (h->st) cudaStreamDestroy(h->st);
+    if (!h->root) {
+        if (h->pin) cudaFreeHost(h->pin);
+        if (h->d_small) cudaFree(h->d_small);
+        if (h->d_chain) cudaFree(h->d_chain);
+        for (auto &e : h->ev) if (e) cudaEventDestroy(e);
+        if (h->fork) cudaEventDestroy(h->fork);
+        if (h->join) cudaEventDestroy(h->join);
+        if (h->st2) cudaStreamDestroy(h->st2);
+        if (h->st) cudaStreamDestroy(h->st);
+    }
     delete h;
 }
 
-// share: a handle on the same device whose static tables are used
-int handle_open(const cz_config *cfg, CZ_HANDLE **out, const CZ_HANDLE *share = nullptr) {
+// a handle for a call's re-runs: its own plan and device memory, everything
+// else its owner's (the two never run at the same time)
+CZ_HANDLE *open_sub(CZ_HANDLE *o) {
+    CZ_HANDLE *h = new CZ_HANDLE();
+    h->cfg = o->cfg;
+    h->dev = o->dev;
+    h->sms = o->sms;
+    h->st = o->st; h->st2 = o->st2; h->fork = o->fork; h->join = o->join;
+    std::copy(o->ev, o->ev + 12, h->ev);
+    h->d_small = o->d_small; h->d_chain = o->d_chain; h->n_small = o->n_small;
+    h->root = o->root ? o->root : o;
+    return h;
+}
+
+int handle_open(const cz_config *cfg, CZ_HANDLE **out) {
     if (!out) return CZ_EINVAL;
     *out = nullptr;
     CZ_HANDLE *h = new CZ_HANDLE();
@@ -982,13 +985,7 @@ int handle_open(const cz_config *cfg, CZ_HANDLE **out, const CZ_HANDLE *share = 
     cudaFuncSetAttribute(gfilter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM);
     cudaFuncSetAttribute(gfilter_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     cudaFuncSetAttribute(plabel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    if (share) {
-        h->d_small = share->d_small; h->d_chain = share->d_chain; h->n_small = share->n_small;
-        h->borrowed = true;
-    } else if (!build_static_tables(h)) {
-        handle_close(h);
-        return CZ_ECUDA;
-    }
+    if (!build_static_tables(h)) { handle_close(h); return CZ_ECUDA; }
     *out = h;
     return CZ_OK;
 }
@@ -1068,53 +1065,44 @@ int census_impl(CZ_HANDLE *h, const pw_t *primes, uint32_t n, uint32_t flags, CZ
     if (n == 0) { if (stats) *stats = s; return CZ_OK; }
     if (!primes || !out || ((flags & CZ_A4) && !a4_out)) { h->err = "null buffer"; return CZ_EINVAL; }
     if ((flags & CZ_AUTO) == 0) flags |= CZ_AUTO;
-    h->sub_live = false;
     int rc = plan(h, primes, n, flags, masks, level);
     if (rc) return rc;
+    h->sub_live = false;
     if (out_cap < h->nprof) { h->have_plan = false; h->err = "output capacity below profile count"; return CZ_EINVAL; }
     if (h->gexec) { cudaGraphExecDestroy(h->gexec); h->gexec = nullptr; }
     if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
-    cudaEvent_t t0, t1;
-    cudaEventCreate(&t0); cudaEventCreate(&t1);
-    cudaEventRecord(t0, h->st);
+    cudaEventRecord(h->ev[9], h->st);
     if ((rc = upload(h, &s))) return rc;
-    cudaEventRecord(t1, h->st);
+    cudaEventRecord(h->ev[10], h->st);
     u32 launches = 0;
     if ((rc = enqueue(h, true, launches))) return rc;
-    h->hout.resize(h->nprof);
-    cudaEvent_t t2;
-    cudaEventCreate(&t2);
-    if (h->nprof && !ck(h, cudaMemcpyAsync(h->hout.data(), h->b_out.p, sizeof(OutRecord) * h->nprof,
-                                           cudaMemcpyDeviceToHost, h->st), "d2h"))
-        return CZ_ECUDA;
-    if ((flags & CZ_A4) && !ck(h, cudaMemcpyAsync(a4_out, h->b_a4.p, 4ull * n, cudaMemcpyDeviceToHost, h->st), "d2h a4"))
-        return CZ_ECUDA;
-    cudaEventRecord(t2, h->st);
+    // counters, records, A4 and states come back in one copy
+    const char *pin = static_cast<const char *>((h->root ? h->root : h)->pin);
+    const char *down = static_cast<const char *>(h->b_small.p) + h->down_off;
+    if (!ck(h, cudaMemcpyAsync((void *)pin, down, h->down_bytes, cudaMemcpyDeviceToHost, h->st), "d2h")) return CZ_ECUDA;
+    cudaEventRecord(h->ev[11], h->st);
     if (!ck(h, cudaStreamSynchronize(h->st), "census")) return CZ_ECUDA;
-    cudaEventElapsedTime(&s.ms_h2d, t0, t1);
-    cudaEventElapsedTime(&s.ms_d2h, h->ev[6], t2);
-    cudaEventDestroy(t0); cudaEventDestroy(t1); cudaEventDestroy(t2);
+    auto got = [&](const Buf &b) { return pin + (static_cast<const char *>(b.p) - down); };
+    cudaEventElapsedTime(&s.ms_h2d, h->ev[9], h->ev[10]);
+    cudaEventElapsedTime(&s.ms_d2h, h->ev[6], h->ev[11]);
     read_times(h, &s);
     s.d2h_bytes = sizeof(OutRecord) * h->nprof + ((flags & CZ_A4) ? 4ull * n : 0ull);
     s.n_primes = n; s.n_dense = h->ndense; s.n_sparse = h->nsparse; s.n_profiles = h->nprof;
     s.kernels = launches;
-    {
-        std::vector<ProfState> hs(h->nprof);
-        if (h->nprof) cudaMemcpy(hs.data(), h->b_state.p, sizeof(ProfState) * h->nprof, cudaMemcpyDeviceToHost);
-        for (auto &x : hs) {
-            s.words += x.words; s.completions += x.completions; s.tests += x.tests;
-            s.staged_bytes += 16ull * x.staged16;
-        }
+    const OutRecord *ho = reinterpret_cast<const OutRecord *>(got(h->b_out));
+    h->hout.assign(ho, ho + h->nprof);
+    if (flags & CZ_A4) std::memcpy(a4_out, got(h->b_a4), 4ull * n);
+    const u32 a4err = reinterpret_cast<const u32 *>(got(h->b_counter))[8];
+    const ProfState *hs = reinterpret_cast<const ProfState *>(got(h->b_state));
+    for (u32 g = 0; g < h->nprof; ++g) {
+        s.words += hs[g].words; s.completions += hs[g].completions; s.tests += hs[g].tests;
+        s.staged_bytes += 16ull * hs[g].staged16;
     }
     // records first: a refusal names the prime and its status
     std::vector<u32> fb, rs;
     rc = check_records(h, allow_fallback ? &fb : nullptr, allow_fallback ? &rs : nullptr);
     if (rc) return rc;
-    if (flags & CZ_A4) {
-        u32 a4err = 0;
-        cudaMemcpy(&a4err, P<u32>(h->b_counter) + 8, 4, cudaMemcpyDeviceToHost);
-        if (a4err) { h->err = "refused: A4 point count not certified"; return CZ_EREFUSED; }
-    }
+    if ((flags & CZ_A4) && a4err) { h->err = "refused: A4 point count not certified"; return CZ_EREFUSED; }
     for (u32 g = 0; g < h->nprof; ++g) {
         const OutRecord &o = h->hout[g];
         CZ_RECORD &d = out[g];
@@ -1133,7 +1121,7 @@ int census_impl(CZ_HANDLE *h, const pw_t *primes, uint32_t n, uint32_t flags, CZ
         // speculation was not certified.  Their orders alone are run again with
         // the threshold one lower, and what misses that too without one, on a
         // handle of their own, so this call's plan stays resident for a replay.
-        if (!h->sub && (rc = handle_open(&h->cfg, &h->sub, h))) { h->err = "re-run handle"; return rc; }
+        if (!h->sub) h->sub = open_sub(h);
         std::vector<pw_t> sp;
         std::vector<u32> sm;
         u32 last = 0xFFFFFFFFu;
