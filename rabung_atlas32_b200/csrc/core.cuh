@@ -287,8 +287,9 @@ constexpr u32 CZ_NOGROUP = 1u << 17;     // internal: every sparse profile on it
 // so much more p.  Measured on 40 windows of 61 primes: groups of near primes
 // of at least 1 / 4 / 8 / 12 members 42.4 / 41.7 / 45.8 / 53.4 ms, this cut with
 // a cost of 1/8, 1/5, 1/3 41.2 / 36.7 / 36.7 ms; 37 primes near 7e8 with 1/8,
-// 1/5, 1/3 2.49 / 2.47 / 2.07 ms on the device.
-constexpr double OWN_COST = 1.0 / 3.0, GROUP_FIXED = 2e7;
+// 1/5, 1/3 2.32 / 2.21 / 1.99 ms on the device, 7 primes near 4.2e9 1.99 / 2.13 /
+// 2.93 ms: the line lies between.
+constexpr double OWN_COST = 1.0 / 4.0, GROUP_FIXED = 2e7;
 
 // compared planes and anchor stages of a group: least cost per visited anchor
 // and position of the row.  A stage costs F loads; beta is the bits it is worth
@@ -697,6 +698,12 @@ int upload(CZ_HANDLE *h, cz_stats *s) {
     return CZ_OK;
 }
 
+// rows per threshold epoch of a call with few profiles, at least EPOCH_MIN and
+// EPOCH_PER_PROFILE a profile: the filter's items then fill the GPU (one prime
+// near 2^32: 1024 rows 0.59 ms, 64 a profile 0.41; 3 primes near 4.2e9 with 128,
+// 64, 32 a profile 0.90 / 0.86 / 0.84 ms)
+constexpr u32 EPOCH_MIN = 32, EPOCH_PER_PROFILE = 32;
+
 // enqueue the device work of the current plan on h->st; returns launches
 int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
     cudaStream_t st = h->st;
@@ -809,7 +816,10 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         // (up to 64), so small calls fill the GPU; large calls keep the tuned group
         sa.group = std::max(std::max(1u, h->cfg.cta_per_profile), std::min(64u, grid / std::max(1u, h->nsl)));
         sa.tune.screen = h->cfg.screen;
-        sa.epoch_rows = h->cfg.epoch_rows;
+        // and cuts its rows into shorter epochs, so that there are items for them:
+        // near 2^32 a profile has 8 epochs of 1024 rows and some 5 tiles each
+        const u32 erows = h->cfg.epoch_rows ? h->cfg.epoch_rows : EPOCH_ROWS_DEFAULT;
+        sa.epoch_rows = std::min(erows, std::max(EPOCH_MIN, EPOCH_PER_PROFILE * h->nsl));
         grid = std::min(grid, h->nsl * sa.group);
         sparse_kernel<<<grid, SPARSE_WARPS * 32, TILE_WORDS * 4u, st>>>(sa);
         ++launches;
