@@ -76,7 +76,7 @@ constexpr u32 G_TILE3 = G_TILE_WORDS / 3u / 4u * 4u * 8u;    // byte offset of p
 constexpr u32 G_OFFS = G_UNITS * G_TMAX / 8u; // 16-byte words of an offset table (16-bit tile positions)
 constexpr u32 G_SMEM = 8u * G_TILE_WORDS + 32u * G_OFFS;   // dynamic shared memory of the filter
 constexpr u32 G_PAD = 384;                // guard indices at both ends of a class array
-constexpr int G_SCR_CAP = 64;             // queued anchors per warp (< 32 + one step of 32)
+constexpr int G_SCR_CAP = 96;             // queued anchors per warp (< 32 + two rows' step of 32)
 constexpr int G_CAND_CAP = 48;            // queued candidates per warp (<= 16 + one round of 32)
 
 struct GroupDesc {
@@ -481,7 +481,9 @@ struct GSlot {
     u32 unit;                     // next unit to claim
     u32 base[G_TMAX], S[G_TMAX], L[G_TMAX];
     u32 lim[G_ROWS], first[G_ROWS], spi[G_ROWS], nb[G_ROWS];
-    uint4 units[G_UNITS];         // row d, numerator of rank 0, ranks | last index << 16, ny | spacing << 16
+    // narrow: row d, numerator of rank 0, ranks | last index << 16, ny | spacing << 16;
+    // wide: row d, numerator of rank 0, ranks of d | ranks of d + 6 << 16, 0
+    uint4 units[G_UNITS];
     unsigned long long full, empty;
 };
 
@@ -677,51 +679,51 @@ __device__ __noinline__ void gflush(const GShared &sh, const GroupDesc &G, GWarp
     __syncwarp();
 }
 
-// screen the first `count` (<= 32) of n queued anchors, one per lane, and
-// queue the members that survive
+// screen the n queued anchors, 32 at a time and one per lane, and queue the
+// members that survive; fewer than 32 stay (none with `all`).  Returns how many.
 template <int F>
-__device__ __noinline__ void gscreen_batch(const GShared &sh, const GroupDesc &G, GWarp &w, u32 n, u32 count,
-                                           u32 lane) {
-    u32 keep = 0u, b = 0u, d = 0u;
-    if (lane < count) {
-        const GEnt e = w.scr[lane];
-        b = e.b;
-        d = e.d;
-        keep = gscreen<F>(G, sh.a.planes + G.off, sh.a.planes2 + G.off2, b, d, e.alive);
-    }
-    __syncwarp();
-    GEnt mv{0u, 0u, 0u};
-    const bool has = lane < n - count;                     // at most 32 stay
-    if (has) mv = w.scr[count + lane];
-    __syncwarp();
-    if (has) w.scr[lane] = mv;
+__device__ __noinline__ u32 gscreen_batch(const GShared &sh, const GroupDesc &G, GWarp &w, u32 n, bool all, u32 lane) {
     u32 nc = w.ncand;
     __syncwarp();
-    for (u32 bal = __ballot_sync(0xFFFFFFFFu, keep != 0u); bal; bal = __ballot_sync(0xFFFFFFFFu, keep != 0u)) {
-        if (keep) {
-            const u32 mb = __ffs(keep) - 1u;
-            keep &= keep - 1u;
-            w.cand[nc + __popc(bal & ((1u << lane) - 1u))] = GCand{b, (d << 5) | mb};
+    while (n >= 32u || (all && n)) {
+        // the last entries: the others need no move
+        const u32 count = min(32u, n);
+        n -= count;
+        u32 keep = 0u, b = 0u, d = 0u;
+        if (lane < count) {
+            const GEnt e = w.scr[n + lane];
+            b = e.b;
+            d = e.d;
+            keep = gscreen<F>(G, sh.a.planes + G.off, sh.a.planes2 + G.off2, b, d, e.alive);
         }
-        nc += __popc(bal);
-        __syncwarp();
-        if (nc > 16u) {
-            const u32 count = min(32u, nc);
-            gflush(sh, G, w, nc, count, lane);
-            nc -= count;
+        for (u32 bal = __ballot_sync(0xFFFFFFFFu, keep != 0u); bal; bal = __ballot_sync(0xFFFFFFFFu, keep != 0u)) {
+            if (keep) {
+                const u32 mb = __ffs(keep) - 1u;
+                keep &= keep - 1u;
+                w.cand[nc + __popc(bal & ((1u << lane) - 1u))] = GCand{b, (d << 5) | mb};
+            }
+            nc += __popc(bal);
+            __syncwarp();
+            if (nc > 16u) {
+                const u32 m = min(32u, nc);
+                gflush(sh, G, w, nc, m, lane);
+                nc -= m;
+            }
         }
     }
+    __syncwarp();
     if (lane == 0) w.ncand = nc;
     __syncwarp();
+    return n;
 }
 
 // the F planes' words of all T stages for one anchor per lane.  ad[j] is the
 // lane's shared byte address of stage j in the tile's planes 0 and 1, ad3[j]
 // (F = 3) in its plane 2; disp (indices) is a compile-time displacement.
-template <int F, int T>
+template <int F, int T, int J0 = 0>
 __device__ __forceinline__ void gwords(const u32 *ad, const u32 *ad3, u32 disp, u32 (*x)[T]) {
 #pragma unroll
-    for (int j = 0; j < T; ++j) {
+    for (int j = J0; j < T; ++j) {
         if constexpr (F == 1) {
             x[0][j] = lds32(ad[j] + 4u * disp);
         } else {
@@ -758,12 +760,15 @@ __device__ __forceinline__ u32 gtest(const u32 *ad, const u32 *ad3, u32 disp) {
     gwords<F, T>(ad, ad3, disp, x);
     return gagree<F, T>(x);
 }
-// two steps, 32 anchor indices apart, with all their loads in flight together
+// the same anchors (same numerators) of two rows: the base words are read once
 template <int F, int T>
-__device__ __forceinline__ void gtest2(const u32 *ad, const u32 *ad3, u32 disp, u32 &r0, u32 &r1) {
+__device__ __forceinline__ void gtest2(const u32 *ad, const u32 *ad3, const u32 *bd, const u32 *bd3, u32 disp, u32 &r0,
+                                       u32 &r1) {
     u32 x[F][T], y[F][T];
     gwords<F, T>(ad, ad3, disp, x);
-    gwords<F, T>(ad, ad3, disp + 32u, y);
+    gwords<F, T, 1>(bd, bd3, disp, y);
+#pragma unroll
+    for (int f = 0; f < F; ++f) y[f][0] = x[f][0];
     r0 = gagree<F, T>(x);
     r1 = gagree<F, T>(y);
 }
@@ -779,74 +784,76 @@ __device__ __forceinline__ bool gqueue(GEnt *scr, u32 &n, u32 b, u32 d, u32 aliv
     return n >= 32u;
 }
 
-// one unit (row, class) from rank `i` on: false when a full batch waits for
-// the screen first (the caller screens with none of this state live and
-// resumes at i), true when the unit is done.  A wide unit's ranks are
-// consecutive indices of its chunk; a narrow unit's run over the indices of
-// its bands, ny a band, bands spi indices apart.
+// byte addresses of a unit's stages: tabulated positions, from index l0 on
+template <int F, int T>
+__device__ __forceinline__ void gaddresses(const uint4 *of, u32 tile, u32 l0, u32 *ad, u32 *ad3) {
+    constexpr u32 A = F == 1 ? 4u : 8u;                    // bytes of planes 0 and 1 per index
+    u32 v[8];
+    const uint4 p = of[0];
+    v[0] = p.x; v[1] = p.y; v[2] = p.z; v[3] = p.w;
+    if constexpr (T > 8) {
+        const uint4 r = of[1];
+        v[4] = r.x; v[5] = r.y; v[6] = r.z; v[7] = r.w;
+    }
+    const u32 t0 = tile + l0 * A, t3 = tile + G_TILE3 + l0 * 4u;
+#pragma unroll
+    for (int j = 0; j < T; ++j) {
+        const u32 k = (j & 1) ? v[j >> 1] >> 16 : v[j >> 1] & 0xFFFFu;
+        ad[j] = t0 + k * A;
+        if constexpr (F == 3) ad3[j] = t3 + k * 4u;
+    }
+}
+
+// One unit from rank `i` on: false when a full batch waits for the screen
+// first (the caller screens with none of this state live and resumes at i),
+// true when the unit is done.  A wide unit is a class of two rows d, d + 6,
+// whose bands start together: ranks are the chunk's consecutive indices, the
+// anchors' own words are read once for both rows (measured on 128 primes from
+// 4.2e9: two steps of one row 14.8 ms, one step of two rows 13.7).  A narrow unit
+// is a class of one row: ranks run over the indices of its bands, ny a band, spi apart.
 template <int F, int T>
 __device__ __forceinline__ bool gunit(const uint4 U, const uint4 *of, u32 tile, u32 live, u32 &i, GWarp &w, u32 &n,
                                       u32 lane) {
-    const u32 cnt = U.z & 0xFFFFu;
-    constexpr u32 A = F == 1 ? 4u : 8u;                    // bytes of planes 0 and 1 per index
+    constexpr u32 A = F == 1 ? 4u : 8u;
     u32 ad[T], ad3[F == 3 ? T : 1];
-    {
-        u32 v[8];
-        const uint4 p = of[0];
-        v[0] = p.x; v[1] = p.y; v[2] = p.z; v[3] = p.w;
-        if constexpr (T > 8) {
-            const uint4 r = of[1];
-            v[4] = r.x; v[5] = r.y; v[6] = r.z; v[7] = r.w;
-        }
-        const u32 l0 = U.w ? 0u : i + lane, t0 = tile + l0 * A, t3 = tile + G_TILE3 + l0 * 4u;
-#pragma unroll
-        for (int j = 0; j < T; ++j) {
-            const u32 k = (j & 1) ? v[j >> 1] >> 16 : v[j >> 1] & 0xFFFFu;
-            ad[j] = t0 + k * A;
-            if constexpr (F == 3) ad3[j] = t3 + k * 4u;
-        }
-    }
     if (U.w == 0u) {
+        const u32 ca = U.z & 0xFFFFu, cb = U.z >> 16, most = max(ca, cb), least = min(ca, cb);
+        u32 bd[T], bd3[F == 3 ? T : 1];
+        gaddresses<F, T>(of, tile, i + lane, ad, ad3);
+        gaddresses<F, T>(of + G_TMAX / 8u, tile, i + lane, bd, bd3);
         u32 b = U.y + 6u * (i + lane);
-        // pairs of full steps, two pairs per address update (the displacements
-        // are constants): a pair's loads and logic are independent.  A pair whose
-        // first step fills the queue is cut there, the second is tested again.
         for (;;) {
 #pragma unroll
-            for (u32 h = 0; h < 4u; h += 2u) {
-                if (i + 64u > cnt) {                       // the last one or two steps, maybe partial
-                    if (i < cnt) {
-                        u32 alive = gtest<F, T>(ad, ad3, 32u * h) & live;
-                        if (i + lane >= cnt) alive = 0u;
-                        i += 32u;
-                        if (gqueue(w.scr, n, b + 192u * h, U.x, alive, lane)) return i >= cnt;
-                    }
-                    if (i < cnt) {
-                        u32 alive = gtest<F, T>(ad, ad3, 32u * (h + 1u)) & live;
-                        if (i + lane >= cnt) alive = 0u;
-                        i += 32u;
-                        gqueue(w.scr, n, b + 192u * (h + 1u), U.x, alive, lane);
-                    }
-                    return true;
-                }
+            for (u32 h = 0; h < 2u; ++h) {                 // the second step's displacement is a constant
                 u32 x0, x1;
-                gtest2<F, T>(ad, ad3, 32u * h, x0, x1);
+                gtest2<F, T>(ad, ad3, bd, bd3, 32u * h, x0, x1);
                 x0 &= live;
                 x1 &= live;
-                i += 64u;
-                if (__any_sync(0xFFFFFFFFu, (x0 | x1) != 0u)) {
-                    if (gqueue(w.scr, n, b + 192u * h, U.x, x0, lane)) { i -= 32u; return false; }
-                    if (gqueue(w.scr, n, b + 192u * (h + 1u), U.x, x1, lane)) return i >= cnt;
+                if (i + 32u > least) {                     // partial in one row or both
+                    if (i + lane >= ca) x0 = 0u;
+                    if (i + lane >= cb) x1 = 0u;
                 }
+                i += 32u;
+                if (__any_sync(0xFFFFFFFFu, (x0 | x1) != 0u)) {
+                    gqueue(w.scr, n, b + 192u * h, U.x, x0, lane);
+                    if (gqueue(w.scr, n, b + 192u * h, U.x + 6u, x1, lane) || n >= 32u) return i >= most;
+                }
+                if (i >= most) return true;
             }
 #pragma unroll
             for (int j = 0; j < T; ++j) {
-                ad[j] += 128u * A;
-                if constexpr (F == 3) ad3[j] += 512u;
+                ad[j] += 64u * A;
+                if (j) bd[j] += 64u * A;
+                if constexpr (F == 3) {
+                    ad3[j] += 256u;
+                    if (j) bd3[j] += 256u;
+                }
             }
-            b += 768u;
+            b += 384u;
         }
     }
+    gaddresses<F, T>(of, tile, 0u, ad, ad3);
+    const u32 cnt = U.z & 0xFFFFu;
     const u32 ny = U.w & 0xFFFFu, spi = U.w >> 16, last = U.z >> 16;
     const float rny = __frcp_rn(__uint2float_rn(ny));
     const u32 k = div_rcp(i + lane, ny, rny);
@@ -887,16 +894,13 @@ __device__ __forceinline__ void gunits(const GShared &sh, GSlot &sl, const uint4
         u = __shfl_sync(0xFFFFFFFFu, u, 0);
         if (u >= nunits) break;
         const uint4 U = sl.units[u];
-        const u32 cnt = U.z & 0xFFFFu;
+        const u32 cnt = (U.z & 0xFFFFu) + (U.w ? 0u : U.z >> 16);
         if (cnt == 0u) continue;
         words += cnt;
         u32 i = 0;
         for (;;) {
-            const bool done = gunit<F, T>(U, offs + u * (G_TMAX / 8u), tile, live, i, w, n, lane);
-            if (n >= 32u) {
-                gscreen_batch<F>(sh, sl.G, w, n, 32u, lane);
-                n -= 32u;
-            }
+            const bool done = gunit<F, T>(U, offs + u * (U.w ? 1u : 2u) * (G_TMAX / 8u), tile, live, i, w, n, lane);
+            if (n >= 32u) n = gscreen_batch<F>(sh, sl.G, w, n, false, lane);
             if (done) break;
         }
     }
@@ -944,9 +948,9 @@ __device__ __forceinline__ void gfail(const GFilterArgs &a, const GroupDesc &G, 
 // a warp leaves its group: queues, counters and errors
 __device__ __noinline__ void gleave(const GShared &sh, const GroupDesc &G, GWarp &w, u32 n, u32 lane) {
     if (n) {
-        if (G.F == 1u) gscreen_batch<1>(sh, G, w, n, n, lane);
-        else if (G.F == 2u) gscreen_batch<2>(sh, G, w, n, n, lane);
-        else gscreen_batch<3>(sh, G, w, n, n, lane);
+        if (G.F == 1u) gscreen_batch<1>(sh, G, w, n, true, lane);
+        else if (G.F == 2u) gscreen_batch<2>(sh, G, w, n, true, lane);
+        else gscreen_batch<3>(sh, G, w, n, true, lane);
     }
     const u32 nc = w.ncand;
     if (nc) gflush(sh, G, w, nc, nc, lane);
@@ -1061,20 +1065,28 @@ __device__ __noinline__ bool gstage(GShared &sh, GSlot &sl, unsigned short *offs
     }
     __syncwarp();
     // units: their ranks (a narrow unit's rank 0 is its first band's first index)
-    const u32 nunits = (it.nrows + 5u) / 6u * 24u;
+    const u32 nunits = it.wide ? (it.nrows + 11u) / 12u * 24u : (it.nrows + 5u) / 6u * 24u;
     for (u32 u = lane; u < nunits; u += 32u) {
-        const u32 blk = u / 24u, e = G_UNIT[u - 24u * blk], row = 6u * blk + (e >> 4), c = e & 15u, d = it.d0 + row;
-        uint4 U = make_uint4(d, 0u, 0u, 0u);
-        if (row < it.nrows && d) {
-            const u32 lim = sl.lim[row];
-            if (it.wide) {
-                // the chunk's part of the band [c_k, c_k + d), up to lim
-                const i32 len = min(min((i32)(6u * it.W), (i32)d - (i32)(6u * it.x)), (i32)lim + 1 - 6 * it.i0);
-                U.y = 6u * (u32)it.i0 + c;
-                U.z = len > (i32)c ? ((u32)len - c + 5u) / 6u : 0u;
-            } else if (sl.nb[row]) {
+        const u32 blk = u / 24u, e = G_UNIT[u - 24u * blk], c = e & 15u;
+        uint4 U = make_uint4(0u, 0u, 0u, 0u);
+        if (it.wide) {
+            // the chunk's part of the bands [c_k, c_k + d), up to lim, of rows d and d + 6
+            const u32 row = 12u * blk + (e >> 4);
+            U.x = it.d0 + row;
+            U.y = 6u * (u32)it.i0 + c;
+#pragma unroll
+            for (u32 h = 0; h < 2u; ++h) {
+                if (row + 6u * h >= it.nrows) continue;
+                const i32 len = min(min((i32)(6u * it.W), (i32)(U.x + 6u * h) - (i32)(6u * it.x)),
+                                    (i32)sl.lim[row + 6u * h] + 1 - 6 * it.i0);
+                if (len > (i32)c) U.z |= ((u32)len - c + 5u) / 6u << (16u * h);
+            }
+        } else {
+            const u32 row = 6u * blk + (e >> 4), d = it.d0 + row;
+            U.x = d;
+            if (row < it.nrows && d && sl.nb[row]) {
                 // indices of the class in a band (6 | c_k); without spacing: up to the tile's end
-                const u32 spi = sl.spi[row], first = sl.first[row];
+                const u32 lim = sl.lim[row], spi = sl.spi[row], first = sl.first[row];
                 const u32 ny = spi ? (d > c ? (d - c + 5u) / 6u : 0u) : it.W - first;
                 U.y = 6u * ((u32)it.i0 + first) + c;
                 const u32 cnt = sl.nb[row] * ny;
@@ -1086,7 +1098,9 @@ __device__ __noinline__ bool gstage(GShared &sh, GSlot &sl, unsigned short *offs
         }
         sl.units[u] = U;
     }
-    // offsets (stage_off): lane (row, j) divides j d by 6 once for the row's classes
+    // offsets (stage_off): lane (row, j) divides j d by 6 once for the row's
+    // classes.  A wide unit's two rows follow each other; where the second is
+    // past the item's rows, it reads as the first (its ranks are none).
     for (u32 k = lane, n = it.nrows * t; k < n; k += 32u) {
         const u32 row = k / t, j = k - row * t, sj = it.wide ? j : 0u;
         const u32 blk = row / 6u, m6 = row - 6u * blk, e = j * (it.d0 + row), q6 = e / 6u;
@@ -1094,9 +1108,13 @@ __device__ __noinline__ bool gstage(GShared &sh, GSlot &sl, unsigned short *offs
         const i32 at = (i32)(sl.base[sj] + sl.first[row] + (u32)it.i0 + I0 - sl.S[sj]) - (i32)q6;
         const u32 u0 = (u32)(0x120F0B080200ull >> (8u * m6)) & 0xFFu;          // first slot of the row: 0 2 8 11 15 18
         const u32 u1 = m6 == 5u ? 24u : (u32)(0x120F0B080200ull >> (8u * m6 + 8u)) & 0xFFu;
+        const bool twice = it.wide && !(blk & 1u) && row + 6u >= it.nrows;
         for (u32 u = u0; u < u1; ++u) {
             const i32 cc = (i32)(G_UNIT[u] & 15u) - rho;
-            offs[(24u * blk + u) * G_TMAX + j] = (unsigned short)(at + cc * Lj + (cc < 0 ? 6 * Lj - 1 : 0));
+            const unsigned short o = (unsigned short)(at + cc * Lj + (cc < 0 ? 6 * Lj - 1 : 0));
+            const u32 slot = it.wide ? 2u * (24u * (blk >> 1) + u) + (blk & 1u) : 24u * blk + u;
+            offs[slot * G_TMAX + j] = o;
+            if (twice) offs[(slot + 1u) * G_TMAX + j] = o;
         }
     }
     if (lane == 0) {
