@@ -125,11 +125,11 @@ struct CZ_HANDLE {
     std::vector<GroupDesc> hgroups;     // profiles filtered 32 per word (group.cuh)
     std::vector<RowGroup> hrgs;
     std::vector<u32> hitem0;
-    std::vector<uint2> hjobs;
+    std::vector<LabelJob> hjobs;
     u32 n = 0, nprof = 0, ndense = 0, nsparse = 0, nchunks = 0, nsl = 0, ndl = 0;
     u32 ntable = 0;                     // sparse primes with a profile outside the groups (table_kernel)
     bool tab_split = false;             // few of them: labels from the label matrix, several CTAs a prime
-    u32 lab_stride = 0, gmaxB = 0, lab_smem = 0;
+    u32 gmaxB = 0, gmaxq = 0, lab_smem = 0;
     u32 table_smem = 0, dense_smem = 0;
     u32 flags = 0;
     bool have_plan = false;
@@ -242,7 +242,7 @@ u32 qspec_for(const cz_config &c, double lg_p, u32 r, bool allow, u32 level) {
 // primes near 7e4 take 0.53 ms with the scan's own powers and 0.31 ms with kept
 // labels, 400 near 2e4 the same either way (0.39 ms).  Returns the pool's size
 // in labels.
-constexpr u64 DENSE_LABEL_MIN_P = 1u << 16, DENSE_LABEL_WORDS = 1ull << 31;
+constexpr u64 DENSE_LABEL_MIN_P = 1u << 16, DENSE_LABEL_WORDS = 1ull << 30;
 u64 plan_dense_labels(CZ_HANDLE *h) {
     h->h_dlaboff.clear();
     h->h_dlabp.assign(1, 0u);
@@ -380,9 +380,8 @@ u32 group_items(GroupDesc &G, std::vector<RowGroup> &rgs) {
 // row of prime i in the call's label matrix, at least nq labels long
 u32 need_labels(CZ_HANDLE *h, u32 i, u32 nq) {
     PrimeDesc &P = h->hp[i];
-    if (P.job == 0xFFFFFFFFu) { P.job = (u32)h->hjobs.size(); h->hjobs.push_back(make_uint2(i, 0u)); }
-    h->hjobs[P.job].y = std::max(h->hjobs[P.job].y, nq);
-    h->lab_stride = std::max(h->lab_stride, (nq + 63u) & ~63u);     // rows hold whole 16-byte loads of labels
+    if (P.job == 0xFFFFFFFFu) { P.job = (u32)h->hjobs.size(); h->hjobs.push_back(LabelJob{i, 0u, 0ull}); }
+    h->hjobs[P.job].nq = std::max(h->hjobs[P.job].nq, nq);
     return P.job;
 }
 
@@ -492,6 +491,7 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
         G.pwoff = pwwords;
         pwwords += (u64)G.nq * G.np;
         h->gmaxB = std::max(h->gmaxB, G.B);
+        h->gmaxq = std::max(h->gmaxq, G.nq);
     }
     h->hitem0.push_back(items);
 }
@@ -516,7 +516,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
     h->h_didx.clear(); h->h_sidx.clear(); h->h_slist.clear(); h->h_dlist.clear();
     h->h_chunk.assign(1, 0u); h->h_summp.clear();
     h->hgroups.clear(); h->hrgs.clear(); h->hitem0.clear(); h->hjobs.clear();
-    h->nsparse = 0; h->gmaxB = 0; h->lab_stride = 0;
+    h->nsparse = 0; h->gmaxB = 0; h->gmaxq = 0;
     u64 plane_words = 0;
     u32 max_slots_t = 8, max_slots_d = 8, max_nq = 0;
     u64 summ_slots = 0;
@@ -640,6 +640,8 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
     }
     h->lab_smem = max_slots_t * (u32)(sizeof(pw_t) + 2u) + 16u;
     const u64 dlab = plan_dense_labels(h);
+    u64 labels = 0;
+    for (LabelJob &J : h->hjobs) { J.off = labels; labels += (J.nq + 63u) & ~63u; }
     h->table_smem = max_slots_t * (u32)(sizeof(pw_t) + 2u) + 8u + max_nq * 2u + 16u;
     if (h->table_smem > TABLE_DYN_SMEM) {
         h->err = "table shared memory above the per-block limit";
@@ -665,7 +667,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
     place(at_big, big, h->b_planes, plane_words * 4ull);
     place(at_big, big, h->b_summ, sizeof(Summ) * summ_slots);
     place(at_big, big, h->b_dlab, 2ull * dlab);
-    place(at_big, big, h->b_lab, 2ull * h->lab_stride * h->hjobs.size());
+    place(at_big, big, h->b_lab, 2ull * labels);
     place(at_big, big, h->b_pw, 4ull * pwwords);
     place(at_big, big, h->b_gplanes, 4ull * gwords);
     place(at_big, big, h->b_gplanes2, 4ull * gwords2);
@@ -737,10 +739,9 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         LabelArgs la;
         la.primes = P<PrimeDesc>(h->b_primes);
         la.state = P<ProfState>(h->b_state);
-        la.jobs = P<uint2>(h->b_jobs);
+        la.jobs = P<LabelJob>(h->b_jobs);
         la.nchunk = std::max(2u, std::min(96u, 8u * (u32)h->sms / njobs));
         la.lab = P<unsigned short>(h->b_lab);
-        la.stride = h->lab_stride;
         la.small_primes = h->d_small;
         plabel_kernel<<<njobs * la.nchunk, 256, h->lab_smem, st>>>(la);
         ++launches;
@@ -750,13 +751,13 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         ga.groups = P<GroupDesc>(h->b_groups);
         ga.ngroups = ngroups;
         ga.lab = P<unsigned short>(h->b_lab);
-        ga.stride = h->lab_stride;
+        ga.jobs = P<LabelJob>(h->b_jobs);
         ga.pw = P<u32>(h->b_pw);
         ga.planes = P<u32>(h->b_gplanes);
         ga.planes2 = P<u32>(h->b_gplanes2);
         ga.chain = h->d_chain;
         ga.small_primes = h->d_small;
-        const u32 qblk = h->lab_stride / 32u;
+        const u32 qblk = (h->gmaxq + 31u) / 32u;
         gpack_kernel<<<(ngroups * qblk + 7u) / 8u, 256, 0, st>>>(ga, qblk);
         gtable_low_kernel<<<ngroups, 512, 0, st>>>(ga);
         launches += 2;
@@ -779,7 +780,7 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         ta.chain = h->d_chain;
         ta.chain_limit = CHAIN_LIMIT;
         ta.lab = h->tab_split ? P<unsigned short>(h->b_lab) : nullptr;
-        ta.lab_stride = h->lab_stride;
+        ta.jobs = P<LabelJob>(h->b_jobs);
         ta.nchunk = h->tab_split ? std::max(1u, std::min(64u, 2u * (u32)h->sms / h->ntable)) : 1u;
         const u32 grid = ta.lab ? h->ntable * ta.nchunk : std::min<u32>(h->ntable, (u32)h->sms);
         table_kernel<<<grid, TABLE_THREADS, ta.lab ? 0u : h->table_smem, st>>>(ta);

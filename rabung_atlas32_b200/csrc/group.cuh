@@ -49,9 +49,12 @@
 // the words of the anchors' positions b - j d for 48 neighbouring rows d, whose
 // segments nearly coincide, so a staged word is used about 30 times.  Measured
 // on 128 primes from 4.2e9 (421 profiles): 29.9 ms on per-profile planes
-// (sparse.cuh) -> 13.5 ms, load path 76 % busy in the stage loop, plus 1.2 ms
-// for the profiles left over; a block of 4096 primes below 2^32: 757 -> 422 ms,
-// its tables 71 -> 9.3 ms.  Members of a group should be many: the cost does not
+// (sparse.cuh) -> 13.7 ms, load path 74 % and issue 64 % busy, 5.0e12 words
+// compared a second of the 9.3e12 the load path could deliver; a block of 4096
+// primes below 2^32: 757 -> 375 ms, its tables 71 -> 7 ms.  18 testing warps with
+// 96 registers: 14, 16, 20, 22, 26 warps take 16.3, 15.4, 16.1, 16.0, 16.0 ms
+// against 14.8 (before rows were paired), rows per item 24, 36, 72 against 48
+// 16.7, 15.2, 15.6 ms.  Members of a group should be many: the cost does not
 // depend on their number.
 #pragma once
 #include "sparse.cuh"
@@ -140,14 +143,6 @@ CZ_HD void seg_range(const GItem &it, u32 t, u32 j, u32 I0, u32 CL, u32 &S, u32 
     if (b > (i32)CL) b = (i32)CL;                       // a narrow item at the table's end
     S = (u32)a;
     L = (u32)(b - a);
-}
-
-// position in the tile (in indices) of stage j of the anchor at index 0, row
-// d, class c, given the first position and the range of the stage's segment
-CZ_HD u32 stage_off(const GItem &it, u32 d, u32 c, u32 j, u32 I0, u32 base, u32 S, u32 L) {
-    const i32 n = 6 * it.i0 + (i32)c - (i32)(j * d);
-    const i32 i = floor6(n);
-    return base + (u32)(n - 6 * i) * L + (u32)(i + (i32)I0) - S;
 }
 
 // layout of a group's class arrays: every segment of every item starts at an
@@ -240,10 +235,9 @@ template <int R> struct Sliced {
 struct LabelArgs {
     const PrimeDesc *primes;
     ProfState *state;
-    const uint2 *jobs;            // (prime index, primes needed)
+    const LabelJob *jobs;
     u32 nchunk;                   // CTAs per job
-    unsigned short *lab;          // label matrix, one row per job
-    u32 stride;                   // its row length (multiple of 64)
+    unsigned short *lab;          // label pool
     const u32 *small_primes;
 };
 
@@ -253,18 +247,18 @@ struct LabelArgs {
 __global__ void __launch_bounds__(256)
 plabel_kernel(LabelArgs a) {
     extern __shared__ __align__(16) u32 lsm[];
-    const uint2 job = a.jobs[blockIdx.x / a.nchunk];
+    const LabelJob job = a.jobs[blockIdx.x / a.nchunk];
     const u32 chunk = blockIdx.x % a.nchunk;
-    const PrimeDesc P = a.primes[job.x];
+    const PrimeDesc P = a.primes[job.prime];
     if (P.status & ST_ROOT) return;              // refused: its member is masked out of the filter
     const Mont M{P.p, P.pinv, P.one, P.r2};
     const u32 slots = hash_slots(P.m);
     pw_t *keys = reinterpret_cast<pw_t *>(lsm);
     unsigned short *hl = reinterpret_cast<unsigned short *>(keys + slots);
     build_root_hash(keys, hl, slots, M, P.z, P.m);
-    const u32 per = ((job.y + a.nchunk - 1u) / a.nchunk + 63u) & ~63u;
-    const u32 lo = chunk * per, hi = min(job.y, lo + per);
-    unsigned short *row = a.lab + (size_t)(blockIdx.x / a.nchunk) * a.stride;
+    const u32 per = ((job.nq + a.nchunk - 1u) / a.nchunk + 63u) & ~63u;
+    const u32 lo = chunk * per, hi = min(job.nq, lo + per);
+    unsigned short *row = a.lab + job.off;
     u32 bad = 0;
     for (u32 i = lo + threadIdx.x; i < hi; i += 2u * blockDim.x) {
         const u32 i2 = i + blockDim.x;
@@ -287,7 +281,7 @@ struct GTableArgs {
     const GroupDesc *groups;
     u32 ngroups;
     const unsigned short *lab;
-    u32 stride;
+    const LabelJob *jobs;
     u32 *pw;                      // bit-sliced colours of the primes <= B, per group
     u32 *planes, *planes2;        // pools of planes 0, 1 and of planes 2, 3
     const uint2 *chain;
@@ -307,7 +301,7 @@ gpack_kernel(GTableArgs a, u32 nblk) {
     const bool in = lane < G.n;
     uint4 v[4];
     if (in) {
-        const uint4 *row = reinterpret_cast<const uint4 *>(a.lab + (size_t)G.job[lane] * a.stride + i0);
+        const uint4 *row = reinterpret_cast<const uint4 *>(a.lab + a.jobs[G.job[lane]].off + i0);
 #pragma unroll
         for (int k = 0; k < 4; ++k) v[k] = row[k];
     }
@@ -1098,7 +1092,9 @@ __device__ __noinline__ bool gstage(GShared &sh, GSlot &sl, unsigned short *offs
         }
         sl.units[u] = U;
     }
-    // offsets (stage_off): lane (row, j) divides j d by 6 once for the row's
+    // offsets: the tile position of stage j of the anchor at index 0, row d, class
+    // c is that of n = 6 i0 + c - j d, i.e. base + (n mod 6) L + floor(n / 6) + I0 - S
+    // of the stage's segment; lane (row, j) divides j d by 6 once for the row's
     // classes.  A wide unit's two rows follow each other; where the second is
     // past the item's rows, it reads as the first (its ranks are none).
     for (u32 k = lane, n = it.nrows * t; k < n; k += 32u) {

@@ -22,20 +22,10 @@ CZ_HD u32 hash_slots(u32 m) {
 CZ_HD u32 hash_slot(u32 key, u32 bits) { return (key * 0x9E3779B1u) >> (32 - bits); }
 CZ_HD u32 hash_slot(u64 key, u32 bits) { return hash_slot((u32)key ^ (u32)(key >> 32) * 0x85EBCA6Bu, bits); }
 
-// element of exact order m: z = a^((p-1)/m) with z^(m/q) != 1 for each prime
-// q | m (the reference's character_root; only m is factored).
-CZ_HD pw_t find_root_of_order(const Mont &M, pw_t p, u32 m, pw_t e) {
-    if (m == 1) return M.one;
-    for (u32 a = 2; a < p && a < 100000u; ++a) {
-        pw_t z = mpow(to_mont((pw_t)a, M), e, M);
-        bool ok = true;
-        const u32 qs[4] = {2, 3, 5, 7};
-        for (int i = 0; i < 4; ++i)
-            if (m % qs[i] == 0 && mpow(z, m / qs[i], M) == M.one) { ok = false; break; }
-        if (ok) return z;
-    }
-    return 0;
-}
+// one row of a call's label matrix: the labels of the first nq primes for one
+// prime of the call, from label `off` of the pool on (a multiple of 64, so that
+// 32 labels are whole 16-byte loads)
+struct LabelJob { u32 prime, nq; u64 off; };
 
 // Block-cooperative build of the root hash for one prime in shared memory.
 // keys[] must hold hash_slots(m) prime-sized words, labels[] as many u16.

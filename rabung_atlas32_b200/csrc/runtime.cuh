@@ -548,7 +548,7 @@ void admit(cz_server *s) {
         ta.chain = s->h->d_chain;
         ta.chain_limit = CHAIN_LIMIT;
         ta.lab = nullptr;
-        ta.lab_stride = 0;
+        ta.jobs = nullptr;
         ta.nchunk = 1;
         table_kernel<<<std::min<u32>(ta.nsparse, (u32)s->h->sms), TABLE_THREADS, table_smem, st>>>(ta);
         if (cudaStreamSynchronize(st) != cudaSuccess) {

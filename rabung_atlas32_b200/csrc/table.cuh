@@ -62,10 +62,11 @@ struct TableArgs {
     const uint2 *chain;          // chain[n] = (index of q = spf(n) in small_primes | e << 24, n / q^e)
     u32 chain_limit;
     // calls of few primes: labels of the small primes computed beforehand over
-    // the whole GPU (plabel_kernel, row PrimeDesc.job of lab_stride labels), and
+    // the whole GPU (plabel_kernel, job PrimeDesc.job), and
     // nchunk CTAs per prime, each a part of the numerators; nullptr, 1 otherwise
     const unsigned short *lab;
-    u32 lab_stride, nchunk;
+    const LabelJob *jobs;
+    u32 nchunk;
 };
 
 struct TabProf {            // per-profile constants of the CTA's prime
@@ -99,7 +100,7 @@ table_kernel(TableArgs a) {
         pw_t *keys = reinterpret_cast<pw_t *>(tsm);
         unsigned short *hl = reinterpret_cast<unsigned short *>(keys + slots);
         unsigned short *own = hl + slots + 4u;
-        const unsigned short *plab = a.lab ? a.lab + (size_t)P.job * a.lab_stride : own;
+        const unsigned short *plab = a.lab ? a.lab + a.jobs[P.job].off : own;
         if (!a.lab) build_root_hash(keys, hl, slots, M, P.z, P.m);
         const u32 KS = (P.B + 1u + 31u) / 32u + 1u;            // steps: n in [0, 32*KS)
         const u32 nmax = 32u * KS;
