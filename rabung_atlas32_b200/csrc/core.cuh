@@ -167,55 +167,50 @@ bool ensure(CZ_HANDLE *h, Buf &b, size_t bytes) {
 
 template <class T> T *P(Buf &b) { return reinterpret_cast<T *>(b.p); }
 
-bool build_static_tables(CZ_HANDLE *h) {
-    // primes below CHAIN_LIMIT and the prime-power chain: chain[n] =
-    // (index of q = spf(n) | e << 24, n / q^e) with q^e the full power of q in
-    // n, so a walk takes one step per distinct prime factor (at most 7 below
-    // 2^20), not one per factor
-    std::vector<u32> spf(CHAIN_LIMIT, 0);
+// primes below CHAIN_LIMIT and the prime-power chain: chain[n] = (index of
+// q = spf(n) | e << 24, n / q^e) with q^e the full power of q in n, so a walk
+// takes one step per distinct prime factor (at most 7 below 2^20), not one per
+// factor.  Constants, made once per process (some 25 ms); each handle copies
+// them to its device.
+struct StaticTables {
     std::vector<u32> primes;
-    for (u32 i = 2; i < CHAIN_LIMIT; ++i) {
-        if (!spf[i]) {
+    std::vector<uint2> chain;
+};
+const StaticTables &static_tables() {
+    static StaticTables t;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        std::vector<u32> spf(CHAIN_LIMIT, 0), index(CHAIN_LIMIT, 0);
+        for (u32 i = 2; i < CHAIN_LIMIT; ++i) {
+            if (spf[i]) continue;
             spf[i] = i;
-            primes.push_back(i);
+            index[i] = (u32)t.primes.size();
+            t.primes.push_back(i);
             if ((u64)i * i < CHAIN_LIMIT)
                 for (u32 j = i * i; j < CHAIN_LIMIT; j += i)
                     if (!spf[j]) spf[j] = i;
         }
-    }
-    std::vector<u32> index(CHAIN_LIMIT, 0);
-    for (u32 k = 0; k < primes.size(); ++k) index[primes[k]] = k;
-    std::vector<uint2> chain(CHAIN_LIMIT);
-    chain[0] = make_uint2(0, 0);
-    chain[1] = make_uint2(0, 1);
-    for (u32 n = 2; n < CHAIN_LIMIT; ++n) {
-        const u32 q = spf[n];
-        u32 m = n, e = 0;
-        while (m % q == 0) { m /= q; ++e; }
-        chain[n] = make_uint2(index[q] | (e << 24), m);     // index < 2^17, e <= 20
-    }
-    h->n_small = (u32)primes.size();
-    if (!ck(h, cudaMalloc(&h->d_small, primes.size() * 4), "cudaMalloc small")) return false;
-    if (!ck(h, cudaMalloc(&h->d_chain, chain.size() * sizeof(uint2)), "cudaMalloc chain")) return false;
-    if (!ck(h, cudaMemcpy(h->d_small, primes.data(), primes.size() * 4, cudaMemcpyHostToDevice), "copy small")) return false;
-    if (!ck(h, cudaMemcpy(h->d_chain, chain.data(), chain.size() * sizeof(uint2), cudaMemcpyHostToDevice), "copy chain")) return false;
-    return true;
+        t.chain.resize(CHAIN_LIMIT);
+        t.chain[0] = make_uint2(0, 0);
+        t.chain[1] = make_uint2(0, 1);
+        for (u32 n = 2; n < CHAIN_LIMIT; ++n) {
+            const u32 q = spf[n];
+            u32 m = n, e = 0;
+            while (m % q == 0) { m /= q; ++e; }
+            t.chain[n] = make_uint2(index[q] | (e << 24), m);     // index < 2^17, e <= 20
+        }
+    });
+    return t;
 }
 
-// the primes below CHAIN_LIMIT, for counting table sizes on the host
-const std::vector<u32> &small_primes() {
-    static std::vector<u32> hs;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        std::vector<char> comp(CHAIN_LIMIT, 0);
-        for (u32 i = 2; i < CHAIN_LIMIT; ++i)
-            if (!comp[i]) {
-                hs.push_back(i);
-                if ((u64)i * i < CHAIN_LIMIT)
-                    for (u32 j = i * i; j < CHAIN_LIMIT; j += i) comp[j] = 1;
-            }
-    });
-    return hs;
+bool build_static_tables(CZ_HANDLE *h) {
+    const StaticTables &t = static_tables();
+    h->n_small = (u32)t.primes.size();
+    if (!ck(h, cudaMalloc(&h->d_small, t.primes.size() * 4), "cudaMalloc small")) return false;
+    if (!ck(h, cudaMalloc(&h->d_chain, t.chain.size() * sizeof(uint2)), "cudaMalloc chain")) return false;
+    if (!ck(h, cudaMemcpy(h->d_small, t.primes.data(), t.primes.size() * 4, cudaMemcpyHostToDevice), "copy small")) return false;
+    if (!ck(h, cudaMemcpy(h->d_chain, t.chain.data(), t.chain.size() * sizeof(uint2), cudaMemcpyHostToDevice), "copy chain")) return false;
+    return true;
 }
 
 u32 q_for(const cz_config &c, u32 r) { return c.q_cap[r] ? c.q_cap[r] : 16u; }
@@ -598,7 +593,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
     h->ndense = (u32)h->h_didx.size();
     h->nchunks = h->h_chunk.back();
     u64 gwords = 0, gwords2 = 0, pwwords = 0;
-    if (h->nsparse && !(flags & (CZ_NOSPEC | CZ_NOGROUP))) plan_groups(h, small_primes(), gwords, gwords2, pwwords);
+    if (h->nsparse && !(flags & (CZ_NOSPEC | CZ_NOGROUP))) plan_groups(h, static_tables().primes, gwords, gwords2, pwwords);
     for (u32 g = 0; g < h->nprof; ++g) {
         ProfDesc &D = h->hprof[g];
         const PrimeDesc &P = h->hp[D.prime];
@@ -617,7 +612,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
     if (h->tab_split)
         for (u32 i : h->h_sidx) {
             const u32 nmax = 32u * ((h->hp[i].B + 1u + 31u) / 32u + 1u);
-            const std::vector<u32> &hs = small_primes();
+            const std::vector<u32> &hs = static_tables().primes;
             need_labels(h, i, (u32)(std::lower_bound(hs.begin(), hs.end(), nmax) - hs.begin()));
         }
     // longest first: the persistent filter hands out profiles in list order,
@@ -635,7 +630,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
     for (u32 i : h->h_sidx) maxB = std::max(maxB, h->hp[i].B);
     if (h->ntable) {
         const u32 nmax = 32u * ((maxB + 1u + 31u) / 32u + 1u);
-        const std::vector<u32> &hs = small_primes();
+        const std::vector<u32> &hs = static_tables().primes;
         max_nq = (u32)(std::lower_bound(hs.begin(), hs.end(), nmax) - hs.begin());
     }
     h->lab_smem = max_slots_t * (u32)(sizeof(pw_t) + 2u) + 16u;
@@ -687,8 +682,10 @@ int upload(CZ_HANDLE *h, cz_stats *s) {
         if (o->pin) cudaFreeHost(o->pin);
         o->pin = nullptr;
         o->pin_cap = 0;
-        if (!ck(h, cudaHostAlloc(&o->pin, total + total / 4, cudaHostAllocDefault), "cudaHostAlloc")) return CZ_ECUDA;
-        o->pin_cap = total + total / 4;
+        // at least a megabyte: a call's re-runs and most later calls fit
+        const size_t want = std::max(total + total / 4, size_t(1) << 20);
+        if (!ck(h, cudaHostAlloc(&o->pin, want, cudaHostAllocDefault), "cudaHostAlloc")) return CZ_ECUDA;
+        o->pin_cap = want;
     }
     // the host plan, laid out as on the device, in one copy
     char *stage = static_cast<char *>(o->pin);
