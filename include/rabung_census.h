@@ -177,7 +177,8 @@ int cz_census_interval(cz_handle *h, uint64_t lo, uint64_t hi, uint32_t flags, u
                        uint32_t *n_profiles, uint32_t *a4_out, cz_stats *stats);
 
 /* ---- serving ---------------------------------------------------------------
- * A server keeps every admitted request resident on the GPU until its records
+ * A server runs requests of up to about 20 ms of filter time at once, together,
+ * and keeps larger ones resident on the GPU until their records
  * are final: the descriptors, per-profile state, colour planes, records and A4
  * of its primes live in device arrays sized when the server opens (colour
  * planes: slots x slot_budget_bytes, capped by free device memory), so a

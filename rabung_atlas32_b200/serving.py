@@ -4,8 +4,10 @@ A request asks for the profiles (and A4) of the `count` consecutive primes
 starting at `lo`.  `Server` drives the library's native serving runtime
 (cz_server_open / cz_submit / cz_next_done / cz_poll, csrc/runtime.cuh):
 
-  * every admitted request stays resident on the GPU (descriptors, state,
-    colour planes, records) until its records are final; admission is by free
+  * a request of up to about 20 ms of filter time runs at once between
+    launches, together with the others like it in one call; a larger one stays
+    resident on the GPU (descriptors, state, colour planes, records) until its
+    records are final; admission is by free
     colour-plane memory and descriptor space;
   * the anchor filter is one persistent kernel over the unfinished profiles of
     all admitted requests; an arrival makes it yield between work items, the
