@@ -114,7 +114,7 @@ struct CZ_HANDLE {
         b_slist, b_dlist, b_dpre, b_out, b_a4, b_counter,
         b_dlab, b_dlaboff, b_dlabp, b_groups, b_rgs, b_item0, b_jobs, b_lab, b_pw, b_gplanes, b_gplanes2;
     // host copies of the current plan
-    std::vector<PrimeDesc> hp;
+    std::vector<PrimeDesc> hp, hp_next;
     std::vector<ProfDesc> hprof;
     std::vector<u32> h_chunk, h_summp, h_didx, h_sidx, h_slist, h_dlist;
     // dense scan: waves of primes whose label arrays fit the pool together
@@ -219,6 +219,22 @@ u32 q_for(const cz_config &c, u32 r) { return c.q_cap[r] ? c.q_cap[r] : 16u; }
 u32 dense_seg(const cz_config &c) {
     const u32 steps = c.dense_steps ? std::min(4096u, std::max(8u, c.dense_steps)) : (u32)DENSE_STEPS;
     return 32u * steps;
+}
+
+// chunks of the dense scan of p
+u32 dense_chunks(pw_t p, u32 seg) {
+    const u32 nh = (u32)((p - 1u) / 2u);                   // < 2^32 for p < 2^33
+    const u32 nseg = (u32)(((u64)nh + seg - 1u) / seg);    // nh + seg wraps 32 bits near 2^33
+    return (nseg + DENSE_WARPS - 1u) / DENSE_WARPS;
+}
+
+// 2: the anchor filter, with its table radius B; 1: the dense scan
+u32 route_of(const cz_config &c, pw_t p, u32 mask, u32 mode, u32 &B) {
+    if (mode != CZ_SPARSE && (mode != CZ_AUTO || p < c.sparse_min_p)) return 1u;
+    u32 Qmax = 0;
+    for (u32 r = 2; r <= 9; ++r)
+        if (mask & (1u << (r - 2))) Qmax = std::max(Qmax, q_for(c, r));
+    return p >= 4096u && Qmax + 1u < p && cover_B(p, Qmax, c.cover_n, B) ? 2u : 1u;
 }
 
 // speculative threshold: floor(log_r p - margin_r), a low quantile of M for
@@ -506,7 +522,38 @@ std::vector<Part> upload_parts(CZ_HANDLE *h) {
 // level: speculative thresholds lowered by so much (re-runs)
 int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = nullptr, u32 level = 0) {
     const cz_config &c = h->cfg;
-    h->hp.assign(n, PrimeDesc{});
+    const u32 mode = flags & CZ_AUTO;
+    const u32 seg = dense_seg(c);
+    // primes, orders and routes first, beside the resident plan: a request
+    // refused here leaves that plan whole, for a replay
+    std::vector<PrimeDesc> &next = h->hp_next;
+    next.assign(n, PrimeDesc{});
+    u64 all_chunks = 0, all_slots = 0;
+    for (u32 i = 0; i < n; ++i) {
+        const pw_t p = primes[i];
+        if (p < 2u || (u64)p >= PW_LIMIT) { h->err = "prime out of domain: " + std::to_string(p); return CZ_EINVAL; }
+        PrimeDesc &P = next[i];
+        P.p = p;
+        P.mask = p > 2u ? mask_of(p) & (masks ? masks[i] : ~0u) : 0u;
+        P.nprof = popc(P.mask);
+        P.job = 0xFFFFFFFFu;
+        if (!P.nprof) continue;
+        P.route = route_of(c, p, P.mask, mode, P.B);
+        if (P.route == 2u) continue;
+        if (mode == CZ_SPARSE) {
+            h->err = "sparse path unsupported for p = " + std::to_string(p);
+            return CZ_EINVAL;
+        }
+        const u32 nch = dense_chunks(p, seg);
+        all_chunks += nch;
+        all_slots += (u64)nch * P.nprof;
+        if (all_chunks > 0xFFFFFFFFull || all_slots > 0xFFFFFFFFull) {
+            h->err = "dense scan too large for one call (chunk index beyond 32 bits)";
+            return CZ_ELIMIT;
+        }
+    }
+    h->have_plan = false;
+    h->hp.swap(next);
     h->hprof.clear();
     h->h_didx.clear(); h->h_sidx.clear(); h->h_slist.clear(); h->h_dlist.clear();
     h->h_chunk.assign(1, 0u); h->h_summp.clear();
@@ -515,36 +562,16 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
     u64 plane_words = 0;
     u32 max_slots_t = 8, max_slots_d = 8, max_nq = 0;
     u64 summ_slots = 0;
-    const u32 mode = flags & CZ_AUTO;
     for (u32 i = 0; i < n; ++i) {
-        const pw_t p = primes[i];
-        if (p < 2u || (u64)p >= PW_LIMIT) { h->err = "prime out of domain: " + std::to_string(p); return CZ_EINVAL; }
         PrimeDesc &P = h->hp[i];
-        P.p = p;
-        P.mask = p > 2u ? mask_of(p) & (masks ? masks[i] : ~0u) : 0u;
+        const pw_t p = P.p;
         P.m = lcm_of_mask(P.mask);
         P.e = P.mask ? (p - 1u) / P.m : 0u;
         P.first_prof = (u32)h->hprof.size();
-        P.nprof = popc(P.mask);
-        P.route = 0;
-        P.job = 0xFFFFFFFFu;
         if (!P.nprof) continue;
-        bool sparse = false;
-        if (mode == CZ_SPARSE) sparse = true;
-        else if (mode == CZ_AUTO) sparse = p >= c.sparse_min_p;
-        u32 B = 0, Qmax = 0;
+        const bool sparse = P.route == 2u;
+        const u32 B = P.B;
         if (sparse) {
-            for (u32 r = 2; r <= 9; ++r)
-                if (P.mask & (1u << (r - 2))) Qmax = std::max(Qmax, q_for(c, r));
-            if (p < 4096u || Qmax + 1u >= p || !cover_B(p, Qmax, c.cover_n, B)) sparse = false;
-            if (!sparse && mode == CZ_SPARSE) {
-                h->err = "sparse path unsupported for p = " + std::to_string(p);
-                return CZ_EINVAL;
-            }
-        }
-        P.route = sparse ? 2u : 1u;
-        if (sparse) {
-            P.B = B;
             // view widths in words, multiples of 4: every view and every tile
             // copy of the filter starts on a 16-byte boundary
             P.K0 = (B + 31u) / 32u + 4u;
@@ -554,14 +581,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
             ++h->nsparse;
             max_slots_t = std::max(max_slots_t, hash_slots(P.m));
         } else {
-            const u32 nh = (u32)((p - 1u) / 2u);           // < 2^32 for p < 2^33
-            const u32 seg = dense_seg(c);
-            const u32 nseg = (u32)(((u64)nh + seg - 1u) / seg);   // nh + seg wraps 32 bits near 2^33
-            const u32 nch = (nseg + DENSE_WARPS - 1u) / DENSE_WARPS;
-            if ((u64)h->h_chunk.back() + nch > 0xFFFFFFFFull || summ_slots + (u64)nch * P.nprof > 0xFFFFFFFFull) {
-                h->err = "dense scan too large for one call (chunk index beyond 32 bits)";
-                return CZ_ELIMIT;
-            }
+            const u32 nch = dense_chunks(p, seg);
             h->h_didx.push_back(i);
             h->h_summp.push_back((u32)summ_slots);
             summ_slots += (u64)nch * P.nprof;
@@ -666,7 +686,6 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
     place(at_big, big, h->b_pw, 4ull * pwwords);
     place(at_big, big, h->b_gplanes, 4ull * gwords);
     place(at_big, big, h->b_gplanes2, 4ull * gwords2);
-    h->have_plan = false;
     if (!ensure(h, h->b_small, small) || !ensure(h, h->b_big, big)) return CZ_ECUDA;
     for (auto &x : at_small) x.first->p = static_cast<char *>(h->b_small.p) + x.second;
     for (auto &x : at_big) x.first->p = static_cast<char *>(h->b_big.p) + x.second;
