@@ -403,7 +403,7 @@ extern "C" int cz_census_dense_noalloc(const uint32_t *primes, uint32_t n, cz_pr
     OutRecord *dO = reinterpret_cast<OutRecord *>(base + L.out);
     const u32 *dpre = ma.prefix_out;
     if (!launch(finalize_kernel, dim3((nprof + FINAL_WARPS - 1) / FINAL_WARPS), dim3(FINAL_WARPS * 32), 0, st, (const PrimeDesc *)dP,
-                (const ProfDesc *)dD, (const ProfState *)dS, dpre, nprof, 0u, dO))
+                (const ProfDesc *)dD, (const ProfState *)dS, dpre, nprof, 0u, (const u32 *)nullptr, 0u, dO))
         return CZ_ECUDA;
     static_assert(sizeof(OutRecord) == sizeof(cz_profile), "record layout");
     if (cudaMemcpyAsync(out, dO, sizeof(OutRecord) * nprof, cudaMemcpyDeviceToHost, st) != cudaSuccess)

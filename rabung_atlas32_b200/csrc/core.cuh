@@ -892,7 +892,8 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
     if (h->nprof) {
         finalize_kernel<<<(h->nprof + FINAL_WARPS - 1) / FINAL_WARPS, FINAL_WARPS * 32, 0, st>>>(
             P<PrimeDesc>(h->b_primes), P<ProfDesc>(h->b_profs), P<ProfState>(h->b_state), P<u32>(h->b_dpre),
-            h->nprof, (h->flags & CZ_VERIFY) ? 1u : 0u, P<OutRecord>(h->b_out));
+            h->nprof, (h->flags & CZ_VERIFY) ? 1u : 0u, P<u32>(h->b_counter) + 4, ngroups ? h->hitem0.back() : 0u,
+            P<OutRecord>(h->b_out));
         ++launches;
     }
     rec(5);

@@ -162,10 +162,10 @@ __device__ __forceinline__ u32 first_fail(u32 n, u32 lane, F pred) {
 // (the serving runtime) or by a warp, whose lanes take the positions.  The key
 // and status words are read through volatile loads: in the serving runtime the
 // last CTA leaving a profile finalises it while other CTAs' atomics on them
-// have just completed.
+// have just completed.  lost: status of the grouped profiles besides their own.
 template <bool WARP>
 __device__ inline void finalize_one(const PrimeDesc *primes, const ProfDesc *profs, const ProfState *state,
-                                    const u32 *dense_prefix, u32 g, u32 verify, OutRecord *out, u32 lane) {
+                                    const u32 *dense_prefix, u32 g, u32 verify, u32 lost, OutRecord *out, u32 lane) {
     const ProfDesc D = profs[g];
     const PrimeDesc P = primes[D.prime];
     const unsigned long long best = *(const volatile unsigned long long *)&state[g].best;
@@ -173,7 +173,7 @@ __device__ inline void finalize_one(const PrimeDesc *primes, const ProfDesc *pro
     const Mont M{P.p, P.pinv, P.one, P.r2};
     const pw_t p = P.p, ex = (p - 1u) / D.r;
     const u32 r = D.r;
-    u32 status = P.status | sstatus;
+    u32 status = P.status | sstatus | (D.grouped ? lost : 0u);
     const u32 Mlen = key_len(best), w = key_witness(best);
     if (best == 0ull && !(D.qspec && P.route == 2u)) status |= ST_VERIFY;
     if (P.route == 2u && D.qspec && Mlen < D.qspec) status |= ST_SPEC;
@@ -222,12 +222,16 @@ constexpr int FINAL_WARPS = 4;     // profiles per CTA
 
 // One warp per profile: certification is M + 2 powers and the prefix another
 // few, independent of one another, so a thread per profile waits for some 40
-// powers in a row (measured: 13,706 profiles 0.15 -> 0.066 ms).
+// powers in a row (measured: 13,706 profiles 0.15 -> 0.066 ms).  *claimed of
+// the group filter's nitems items were handed out; where some were not (every
+// loading warp gave up on a wait), no grouped profile's search was complete.
 __global__ void __launch_bounds__(FINAL_WARPS * 32)
 finalize_kernel(const PrimeDesc *primes, const ProfDesc *profs, const ProfState *state,
-                const u32 *dense_prefix, u32 nprof, u32 verify, OutRecord *out) {
+                const u32 *dense_prefix, u32 nprof, u32 verify, const u32 *claimed, u32 nitems, OutRecord *out) {
     const u32 g = blockIdx.x * FINAL_WARPS + (threadIdx.x >> 5);
-    if (g < nprof) finalize_one<true>(primes, profs, state, dense_prefix, g, verify, out, threadIdx.x & 31u);
+    if (g >= nprof) return;
+    const u32 lost = nitems && *claimed < nitems ? (u32)ST_QUEUE : 0u;
+    finalize_one<true>(primes, profs, state, dense_prefix, g, verify, lost, out, threadIdx.x & 31u);
 }
 
 }  // namespace CZ_NS

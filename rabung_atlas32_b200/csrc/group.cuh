@@ -79,6 +79,12 @@ constexpr u32 G_TILE3 = G_TILE_WORDS / 3u / 4u * 4u * 8u;    // byte offset of p
 constexpr u32 G_OFFS = G_UNITS * G_TMAX / 8u; // 16-byte words of an offset table (16-bit tile positions)
 constexpr u32 G_SMEM = 8u * G_TILE_WORDS + 32u * G_OFFS;   // dynamic shared memory of the filter
 constexpr u32 G_PAD = 384;                // guard indices at both ends of a class array
+#ifndef CZ_GROUP_FULL_TRIES               // bounds of the waits for an item and for a free slot
+#define CZ_GROUP_FULL_TRIES MBAR_SPIN_LIMIT
+#endif
+#ifndef CZ_GROUP_EMPTY_TRIES
+#define CZ_GROUP_EMPTY_TRIES MBAR_SPIN_LIMIT
+#endif
 constexpr int G_SCR_CAP = 96;             // queued anchors per warp (< 32 + two rows' step of 32)
 constexpr int G_CAND_CAP = 48;            // queued candidates per warp (<= 16 + one round of 32)
 
@@ -1129,8 +1135,11 @@ __device__ __noinline__ bool gstage(GShared &sh, GSlot &sl, unsigned short *offs
 // One CTA per SM.  The last two warps each stage items into a slot of their
 // own; the others test the slots in turn, each moving to the next as soon as
 // no unit is left for it, so neither a tile's copy nor an item's end holds the
-// SM up.  Every wait is bounded; a warp whose wait runs out marks its group
-// refused and leaves, and the others' waits run out in turn.
+// SM up.  Every wait is bounded.  A testing warp whose wait runs out marks the
+// group it held and leaves; the loading warps then find their slots taken, mark
+// the group in the slot and the one of the item claimed for it, and leave too,
+// so every item handed out is tested or its group falls back.  Items that
+// nobody claims any more are seen by finalize_kernel.
 __global__ void __launch_bounds__((G_WARPS + 2) * 32, 1)
 gfilter_kernel(GFilterArgs a) {
     extern __shared__ __align__(128) uint4 s_tile[];     // two tiles of G_TILE_WORDS words, two offset tables
@@ -1154,8 +1163,10 @@ gfilter_kernel(GFilterArgs a) {
             u32 g = 0xFFFFFFFFu;
             GItem it;
             const bool has = gclaim(sh.a, lane, g, it);
-            if (r && !mbar_wait_bounded(smem_addr(&sl.empty), (r - 1u) & 1u)) {
+            if (r && !mbar_wait_bounded(smem_addr(&sl.empty), (r - 1u) & 1u, CZ_GROUP_EMPTY_TRIES)) {
                 gfail(sh.a, sl.G, ST_QUEUE, lane);
+                if (has) gfail(sh.a, sh.a.groups[g], ST_QUEUE, lane);
+                mbar_wait_bounded(smem_addr(&sl.full), (r - 1u) & 1u);     // let the copies land before leaving
                 return;
             }
             if (!has) {
@@ -1192,7 +1203,7 @@ gfilter_kernel(GFilterArgs a) {
             prev = 2u;
         }
         GSlot &sl = sh.slot[k];
-        const bool ok = mbar_wait_bounded(smem_addr(&sl.full), (n >> 1) & 1u);
+        const bool ok = mbar_wait_bounded(smem_addr(&sl.full), (n >> 1) & 1u, CZ_GROUP_FULL_TRIES);
         const bool end = ok && sl.group == 0xFFFFFFFFu;
         if (end) ended |= 1u << k;
         if (prev < 2u) {

@@ -455,8 +455,8 @@ __device__ __forceinline__ bool mbar_try_wait(u32 mbar, u32 parity) {
     return ok != 0u;
 }
 // bounded wait for phase `parity` of the tile barrier; false when the limit ran out
-__device__ __forceinline__ bool mbar_wait_bounded(u32 mbar, u32 parity) {
-    for (u32 i = 0; i < MBAR_SPIN_LIMIT; ++i)
+__device__ __forceinline__ bool mbar_wait_bounded(u32 mbar, u32 parity, u32 limit = MBAR_SPIN_LIMIT) {
+    for (u32 i = 0; i < limit; ++i)
         if (mbar_try_wait(mbar, parity)) return true;
     return false;
 }
@@ -743,7 +743,7 @@ __device__ __noinline__ void leave_profile(const SparseArgs &a, const ProfCtx &c
     const u32 left = atomicSub(&st->active, 1u) - 1u;
     const u32 claimed = (u32)*(volatile unsigned long long *)&st->claim;
     if (left != 0u || claimed < c.nitems || atomicCAS(&st->done, 0u, 1u) != 0u) return;
-    finalize_one<false>(a.primes, a.profs, a.state, nullptr, g, a.verify, a.out, 0u);
+    finalize_one<false>(a.primes, a.profs, a.state, nullptr, g, a.verify, 0u, a.out, 0u);
     __threadfence();
     const u32 req = a.profs[g].req;
     if (atomicSub(&a.req_pending[req], 1u) == 1u) {
