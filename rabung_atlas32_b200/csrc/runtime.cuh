@@ -15,16 +15,21 @@
 //    leave their profiles (the claim state stays in device memory) and exit;
 //    the new requests are sieved, planned and tabled on the whole GPU, and the
 //    kernel is relaunched over the old and new unfinished profiles together,
-//    so an arrival waits one work item (tens of microseconds), not a batch;
+//    so an arrival waits for the launch's least time (SRV_MIN_LAUNCH_US or as
+//    long as the joint call before it, at most SRV_CALL_MS) and the work items
+//    in hand (tens of microseconds), not for a batch;
 //  * the last CTA to leave a finished profile certifies and writes its record
 //    and counts the request down; a request's last profile raises its done
 //    flag in mapped host memory, and the scheduler copies its records out
 //    while the kernel keeps running;
 //  * a request of up to about SRV_DIRECT_MS of filter time does not become
-//    resident: in the window it runs at once on the second handle, together with
-//    the others like it in one call, whose profiles form groups across requests
+//    resident: it runs on the second handle, together with others like it in one
+//    call of up to SRV_CALL_MS, whose profiles form groups across requests
 //    (group.cuh; half the time of the per-profile filter and no bookkeeping per
-//    profile).  Only larger ones are worth a launch that yields;
+//    profile).  A window runs one such call; what is left waits for the next
+//    window, which comes after the resident filter has had as much time.  Such
+//    requests need no arena space, so they pass a large one that waits for it.
+//    Only larger ones are worth a launch that yields;
 //  * primes routed to the dense scan (small p), primes whose sparse record
 //    needs the dense re-run, and requests larger than the whole plane arena
 //    (in waves of one slot's planes) are handled by a second handle in the
@@ -85,6 +90,7 @@ struct CzRequest {
     uint32_t lo = 0, count = 0, flags = 0;
     bool given = false;                 // primes supplied by the caller
     bool sieved = false;                // primes found by the device sieve
+    bool small = false;                 // counted in cz_server::small_waiting
     int rc = -1;                        // -1 while pending
     std::string err;
     std::vector<uint32_t> primes;
@@ -109,12 +115,13 @@ constexpr u32 SRV_CAP_PRIMES = 1u << 20;       // resident primes
 constexpr u32 SRV_CAP_PROFILES = 1u << 22;     // resident profiles
 constexpr u32 SRV_CAP_SLOTS = 1u << 16;        // requests in flight
 constexpr int SRV_MIN_LAUNCH_US = 5000;        // a launch runs this long before it yields to arrivals
-// Requests of at most this much modelled filter time run directly in the
-// window, in calls of at most SRV_CALL_MS (what an arrival may have to wait for;
-// a prime near 2^32 takes about SRV_PRIME_MS, in proportion to p, in the groups
-// such calls form).  Measured on 24 requests of 1 to 256 primes submitted
-// together: all resident 46.5 ms, direct 25.8 ms.
-constexpr double SRV_DIRECT_MS = 20.0, SRV_CALL_MS = 40.0, SRV_PRIME_MS = 0.15;
+// Requests of at most SRV_DIRECT_MS of modelled filter time run directly, in
+// calls of at most SRV_CALL_MS, one call a window (a prime near 2^32 takes about
+// SRV_PRIME_MS in the groups such calls form, in proportion to p; an x of the
+// dense scan SRV_X_MS).  The resident filter then runs for as long as that call
+// did, at most SRV_CALL_MS, before it yields again, so a steady stream of small
+// requests leaves it half of the GPU.
+constexpr double SRV_DIRECT_MS = 20.0, SRV_CALL_MS = 40.0, SRV_PRIME_MS = 0.15, SRV_X_MS = 1e-8;
 
 }  // namespace
 
@@ -136,6 +143,8 @@ struct cz_server {
     cudaEvent_t ev_kernel = nullptr;
     bool running = false, yielding = false;
     bool blocked = false;                       // the oldest waiting request needs space in-flight work holds
+    std::deque<CzRequest *> direct;             // small requests taken from `waiting`, next joint calls' work
+    std::chrono::steady_clock::duration min_launch{};   // the resident launch's least time before it yields
     std::chrono::steady_clock::time_point launch_t0, t_yield, t_end;
     bool ended = false;                         // a launch ended and the next has not started
     std::vector<CzRequest *> inflight, repair;
@@ -147,6 +156,8 @@ struct cz_server {
     std::unordered_map<uint64_t, CzRequest *> reqs;
     std::deque<uint64_t> announced;     // completed, not yet returned by cz_next_done
     uint64_t next_id = 1, launches = 0, completed = 0;
+    uint64_t small_waiting = 0;                 // requests in `waiting` that need no arena space
+    uint64_t direct_waiting = 0;                // requests in `direct`
     uint64_t yields = 0, n_respec = 0, n_fallback = 0, n_oversize = 0;
     double ms_drain = 0, ms_window = 0;         // yield flag -> kernel end; kernel end -> relaunch
     bool stop = false;
@@ -321,49 +332,66 @@ double request_ms(const CzRequest *r) {
     return t * (SRV_PRIME_MS / 4294967296.0);
 }
 
-// requests run at once on the second handle, those of like flags together
-void run_direct(cz_server *s, std::vector<CzRequest *> &list) {
-    for (size_t i = 0; i < list.size();) {
-        std::vector<CzRequest *> call, rest;
-        std::vector<uint32_t> ps;
-        const uint32_t flags = list[i]->flags;
-        double ms = 0;
-        for (size_t k = i; k < list.size(); ++k) {
-            CzRequest *r = list[k];
-            const double t = request_ms(r);
-            if (r->flags != flags || (!call.empty() && ms + t > SRV_CALL_MS)) { rest.push_back(r); continue; }
-            ms += t;
-            call.push_back(r);
-            ps.insert(ps.end(), r->primes.begin(), r->primes.end());
-        }
-        std::copy(call.begin(), call.end(), list.begin() + i);
-        i += call.size();
-        std::copy(rest.begin(), rest.end(), list.begin() + i);
-        std::vector<cz_profile> recs;
-        std::vector<uint32_t> a4;
-        cz_stats st{};
-        int rc = census_into(s->aux, ps, flags | CZ_VERIFY, recs, a4, &st);
-        size_t g = 0, k = 0;
-        for (CzRequest *r : call) {
-            if (rc && call.size() > 1) {                   // one of them is refused: each by itself
-                const int own = census_into(s->aux, r->primes, flags | CZ_VERIFY, r->recs, r->a4, &st);
-                finish(s, r, own, own ? s->aux->err : std::string());
-                continue;
-            }
-            if (!rc) {
-                const size_t np = cz_count_profiles(r->primes.data(), (uint32_t)r->primes.size());
-                r->recs.assign(recs.begin() + g, recs.begin() + g + np);
-                g += np;
-                if (flags & CZ_A4) r->a4.assign(a4.begin() + k, a4.begin() + k + r->primes.size());
-                k += r->primes.size();
-            }
-            finish(s, r, rc, rc ? s->aux->err : std::string());
-        }
-        std::lock_guard<std::mutex> lk(s->m);
-        ++s->launches;
-        s->n_respec += st.n_respec;
-        s->n_fallback += st.n_fallback;
+// a request just submitted will run directly (its primes may not be known yet)
+bool small_request(const CzRequest *r) {
+    if ((r->flags & CZ_AUTO) == CZ_DENSE) return false;
+    return (r->given ? request_ms(r) : (double)r->count * r->lo * (SRV_PRIME_MS / 4294967296.0)) <= SRV_DIRECT_MS;
+}
+
+// modelled time of a request's own call: the dense scan of its small primes too
+double call_ms(const cz_server *s, const CzRequest *r) {
+    double x = 0;
+    for (u32 p : r->primes)
+        if (p < s->cfg.sparse_min_p && (r->flags & CZ_AUTO) != CZ_SPARSE) x += 0.5 * (double)p;
+    return request_ms(r) + x * SRV_X_MS;
+}
+
+// one joint call on the second handle: the oldest direct request and, up to
+// SRV_CALL_MS, those of the same flags behind it
+void run_direct(cz_server *s) {
+    s->min_launch = std::chrono::microseconds(SRV_MIN_LAUNCH_US);
+    if (s->direct.empty()) return;
+    const auto t0 = std::chrono::steady_clock::now();
+    std::vector<CzRequest *> call;
+    std::deque<CzRequest *> rest;
+    std::vector<uint32_t> ps;
+    const uint32_t flags = s->direct.front()->flags;
+    double ms = 0;
+    for (CzRequest *r : s->direct) {
+        const double t = r->flags == flags ? call_ms(s, r) : 0.0;
+        if (r->flags != flags || (!call.empty() && ms + t > SRV_CALL_MS)) { rest.push_back(r); continue; }
+        ms += t;
+        call.push_back(r);
+        ps.insert(ps.end(), r->primes.begin(), r->primes.end());
     }
+    s->direct.swap(rest);
+    std::vector<cz_profile> recs;
+    std::vector<uint32_t> a4;
+    cz_stats st{};
+    int rc = census_into(s->aux, ps, flags | CZ_VERIFY, recs, a4, &st);
+    size_t g = 0, k = 0;
+    for (CzRequest *r : call) {
+        if (rc && call.size() > 1) {                       // one of them is refused: each by itself
+            const int own = census_into(s->aux, r->primes, flags | CZ_VERIFY, r->recs, r->a4, &st);
+            finish(s, r, own, own ? s->aux->err : std::string());
+            continue;
+        }
+        if (!rc) {
+            const size_t np = cz_count_profiles(r->primes.data(), (uint32_t)r->primes.size());
+            r->recs.assign(recs.begin() + g, recs.begin() + g + np);
+            g += np;
+            if (flags & CZ_A4) r->a4.assign(a4.begin() + k, a4.begin() + k + r->primes.size());
+            k += r->primes.size();
+        }
+        finish(s, r, rc, rc ? s->aux->err : std::string());
+    }
+    s->min_launch = std::max(s->min_launch, std::min(std::chrono::steady_clock::now() - t0,
+                                                     std::chrono::steady_clock::duration(std::chrono::milliseconds((int)SRV_CALL_MS))));
+    std::lock_guard<std::mutex> lk(s->m);
+    s->direct_waiting = s->direct.size();
+    ++s->launches;
+    s->n_respec += st.n_respec;
+    s->n_fallback += st.n_fallback;
 }
 
 // primes of the requests that name an interval, by one call of the device sieve
@@ -390,7 +418,12 @@ void admit(cz_server *s) {
     std::vector<CzRequest *> batch;
     {
         std::lock_guard<std::mutex> lk(s->m);
-        while (!s->waiting.empty() && batch.size() < 4096) { batch.push_back(s->waiting.front()); s->waiting.pop_front(); }
+        while (!s->waiting.empty() && batch.size() < 4096) {
+            CzRequest *r = s->waiting.front();
+            s->waiting.pop_front();
+            if (r->small) { r->small = false; --s->small_waiting; }
+            batch.push_back(r);
+        }
     }
     if (batch.empty()) return;
     cudaStream_t st = s->h->st;
@@ -407,7 +440,6 @@ void admit(cz_server *s) {
         else
             back.push_back(r);
     };
-    std::vector<CzRequest *> direct;
     sieve_requests(s, batch);
     for (size_t bi = 0; bi < batch.size(); ++bi) {
         CzRequest *r = batch[bi];
@@ -434,7 +466,7 @@ void admit(cz_server *s) {
                 continue;
             }
         }
-        if ((r->flags & CZ_AUTO) != CZ_DENSE && request_ms(r) <= SRV_DIRECT_MS) { direct.push_back(r); continue; }
+        if ((r->flags & CZ_AUTO) != CZ_DENSE && request_ms(r) <= SRV_DIRECT_MS) { s->direct.push_back(r); continue; }
         if (!back.empty()) { back.push_back(r); continue; }
         u32 mode = r->flags & CZ_AUTO;
         if (!mode) mode = CZ_AUTO;
@@ -556,12 +588,10 @@ void admit(cz_server *s) {
             s->inflight.clear();
         }
     }
-    run_direct(s, direct);
     s->blocked = !back.empty();
-    if (!back.empty()) {
-        std::lock_guard<std::mutex> lk(s->m);
-        for (auto it = back.rbegin(); it != back.rend(); ++it) s->waiting.push_front(*it);
-    }
+    std::lock_guard<std::mutex> lk(s->m);
+    for (auto it = back.rbegin(); it != back.rend(); ++it) s->waiting.push_front(*it);
+    s->direct_waiting = s->direct.size();
 }
 
 // launch the filter over the unfinished profiles of every request in flight
@@ -600,18 +630,18 @@ void sched_loop(cz_server *s) {
     cudaSetDevice(s->h->dev);
     for (;;) {
         poll_done(s);
-        bool have_waiting, stopping;
+        bool arrivals, stopping;
         {
             std::lock_guard<std::mutex> lk(s->m);
-            have_waiting = !s->waiting.empty();
+            // while the oldest waits for space still held, only those that need none
+            arrivals = (s->blocked ? s->small_waiting > 0 : !s->waiting.empty()) || !s->direct.empty();
             stopping = s->stop;
         }
         if (s->running) {
-            // yield to arrivals (unless the oldest waits for space still held)
-            // and to dense re-runs, once the launch has run its minimum time
-            const bool ripe = std::chrono::steady_clock::now() - s->launch_t0 >=
-                              std::chrono::microseconds(SRV_MIN_LAUNCH_US);
-            if ((stopping || (ripe && ((have_waiting && !s->blocked) || !s->repair.empty()))) && !s->yielding) {
+            // yield to arrivals, direct requests left over and re-runs, once the
+            // launch has run its minimum time
+            const bool ripe = std::chrono::steady_clock::now() - s->launch_t0 >= s->min_launch;
+            if ((stopping || (ripe && (arrivals || !s->repair.empty()))) && !s->yielding) {
                 cudaMemcpyAsync(s->d_yield, &s->h_flag[0], 4, cudaMemcpyHostToDevice, s->cst);
                 s->yielding = true;
                 s->t_yield = std::chrono::steady_clock::now();
@@ -645,6 +675,7 @@ void sched_loop(cz_server *s) {
         if (stopping) return;
         run_repairs(s);
         admit(s);
+        run_direct(s);
         if (!s->inflight.empty()) {
             launch(s);
             cudaEventRecord(s->ev_kernel, s->h->st);
@@ -657,6 +688,7 @@ void sched_loop(cz_server *s) {
             continue;
         }
         s->ended = false;                              // idle: no window to count
+        if (!s->direct.empty()) continue;
         std::unique_lock<std::mutex> lk(s->m);
         s->cv_work.wait(lk, [s] { return s->stop || !s->waiting.empty(); });
     }
@@ -806,6 +838,8 @@ int cz_submit(cz_server *s, uint32_t lo, uint32_t count, const uint32_t *primes,
         std::lock_guard<std::mutex> lk(s->m);
         if (s->stop) { delete r; return CZ_EINVAL; }
         r->id = s->next_id++;
+        r->small = small_request(r);
+        if (r->small) ++s->small_waiting;
         s->reqs[r->id] = r;
         s->waiting.push_back(r);
         *request_id = r->id;
@@ -859,7 +893,7 @@ int cz_server_info(cz_server *s, uint64_t *batches, uint64_t *completed, uint64_
     std::lock_guard<std::mutex> lk(s->m);
     if (batches) *batches = s->launches;
     if (completed) *completed = s->completed;
-    if (waiting) *waiting = s->waiting.size();
+    if (waiting) *waiting = s->waiting.size() + s->direct_waiting;
     return CZ_OK;
 }
 
@@ -870,7 +904,7 @@ int cz_server_stats(cz_server *s, cz_server_counters *out) {
     out->launches = s->launches;
     out->yields = s->yields;
     out->completed = s->completed;
-    out->waiting = s->waiting.size();
+    out->waiting = s->waiting.size() + s->direct_waiting;
     out->respec_primes = s->n_respec;
     out->fallback_primes = s->n_fallback;
     out->oversize_requests = s->n_oversize;
