@@ -367,12 +367,21 @@ void run_direct(cz_server *s) {
     s->direct.swap(rest);
     std::vector<cz_profile> recs;
     std::vector<uint32_t> a4;
-    cz_stats st{};
-    int rc = census_into(s->aux, ps, flags | CZ_VERIFY, recs, a4, &st);
+    // a call's counters are added before a request of it is announced
+    auto run = [&](const std::vector<uint32_t> &primes, std::vector<cz_profile> &to, std::vector<uint32_t> &toa4) {
+        cz_stats st{};
+        const int own = census_into(s->aux, primes, flags | CZ_VERIFY, to, toa4, &st);
+        std::lock_guard<std::mutex> lk(s->m);
+        ++s->launches;
+        s->n_respec += st.n_respec;
+        s->n_fallback += st.n_fallback;
+        return own;
+    };
+    const int rc = run(ps, recs, a4);
     size_t g = 0, k = 0;
     for (CzRequest *r : call) {
         if (rc && call.size() > 1) {                       // one of them is refused: each by itself
-            const int own = census_into(s->aux, r->primes, flags | CZ_VERIFY, r->recs, r->a4, &st);
+            const int own = run(r->primes, r->recs, r->a4);
             finish(s, r, own, own ? s->aux->err : std::string());
             continue;
         }
@@ -389,9 +398,6 @@ void run_direct(cz_server *s) {
                                                      std::chrono::steady_clock::duration(std::chrono::milliseconds((int)SRV_CALL_MS))));
     std::lock_guard<std::mutex> lk(s->m);
     s->direct_waiting = s->direct.size();
-    ++s->launches;
-    s->n_respec += st.n_respec;
-    s->n_fallback += st.n_fallback;
 }
 
 // primes of the requests that name an interval, by one call of the device sieve
