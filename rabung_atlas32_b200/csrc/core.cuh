@@ -159,10 +159,14 @@ bool ensure(CZ_HANDLE *h, Buf &b, size_t bytes) {
     if (b.p) cudaFree(b.p);
     b.p = nullptr;
     b.cap = 0;
-    size_t want = bytes + bytes / 4;
-    if (!ck(h, cudaMalloc(&b.p, want), "cudaMalloc")) return false;
-    b.cap = want;
-    return true;
+    for (size_t want : {bytes + bytes / 4, bytes}) {       // no slack where memory is short
+        const cudaError_t e = cudaMalloc(&b.p, want);
+        if (e == cudaSuccess) { b.cap = want; return true; }
+        cudaGetLastError();                                // or the next launch check reports it
+        b.p = nullptr;
+        ck(h, e, "cudaMalloc");
+    }
+    return false;
 }
 
 template <class T> T *P(Buf &b) { return reinterpret_cast<T *>(b.p); }
@@ -251,10 +255,11 @@ u32 qspec_for(const cz_config &c, double lg_p, u32 r, bool allow, u32 level) {
 // 210 in memory (dense.cuh), in waves of at most DENSE_LABEL_WORDS 16-bit labels
 // (one prime below 2^33 takes 0.98e9 of them at most).  Where the line lies: 400
 // primes near 7e4 take 0.53 ms with the scan's own powers and 0.31 ms with kept
-// labels, 400 near 2e4 the same either way (0.39 ms).  Returns the pool's size
-// in labels.
+// labels, 400 near 2e4 the same either way (0.39 ms).  The pool stays inside the
+// plane budget; a prime whose labels alone exceed it takes a power for every x.
+// Returns the pool's size in labels (limit 0: no labels).
 constexpr u64 DENSE_LABEL_MIN_P = 1u << 16, DENSE_LABEL_WORDS = 1ull << 30;
-u64 plan_dense_labels(CZ_HANDLE *h) {
+u64 plan_dense_labels(CZ_HANDLE *h, u64 limit) {
     h->h_dlaboff.clear();
     h->h_dlabp.assign(1, 0u);
     h->hwaves.clear();
@@ -277,10 +282,12 @@ u64 plan_dense_labels(CZ_HANDLE *h) {
         if (p >= DENSE_LABEL_MIN_P) {
             const u32 nl = labels_below((u32)((p - 1u) / 2u));
             need = ((u64)nl + DLABEL_HEAD + 7u) & ~7ull;
-            nch = (nl + DLABEL_CHUNK - 1u) / DLABEL_CHUNK;
-            if (used && used + need > DENSE_LABEL_WORDS) close(i);
-            off = used;
-            used += need;
+            if (need <= limit) {
+                nch = (nl + DLABEL_CHUNK - 1u) / DLABEL_CHUNK;
+                if (used && used + need > limit) close(i);
+                off = used;
+                used += need;
+            }
         }
         h->h_dlaboff.push_back(off);
         h->h_dlabp.push_back(h->h_dlabp.back() + nch);
@@ -654,7 +661,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
         max_nq = (u32)(std::lower_bound(hs.begin(), hs.end(), nmax) - hs.begin());
     }
     h->lab_smem = max_slots_t * (u32)(sizeof(pw_t) + 2u) + 16u;
-    const u64 dlab = plan_dense_labels(h);
+    u64 dlab = plan_dense_labels(h, std::min(DENSE_LABEL_WORDS, ((u64)c.plane_budget_mb << 20) / 2u));
     u64 labels = 0;
     for (LabelJob &J : h->hjobs) { J.off = labels; labels += (J.nq + 63u) & ~63u; }
     h->table_smem = max_slots_t * (u32)(sizeof(pw_t) + 2u) + 8u + max_nq * 2u + 16u;
@@ -679,14 +686,25 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
     place(at_small, small, h->b_state, sizeof(ProfState) * h->nprof);
     h->down_bytes = small - h->down_off;
     place(at_small, small, h->b_dpre, 4ull * h->nprof);
-    place(at_big, big, h->b_planes, plane_words * 4ull);
-    place(at_big, big, h->b_summ, sizeof(Summ) * summ_slots);
-    place(at_big, big, h->b_dlab, 2ull * dlab);
-    place(at_big, big, h->b_lab, 2ull * labels);
-    place(at_big, big, h->b_pw, 4ull * pwwords);
-    place(at_big, big, h->b_gplanes, 4ull * gwords);
-    place(at_big, big, h->b_gplanes2, 4ull * gwords2);
-    if (!ensure(h, h->b_small, small) || !ensure(h, h->b_big, big)) return CZ_ECUDA;
+    auto place_big = [&]() {
+        at_big.clear();
+        big = 0;
+        place(at_big, big, h->b_planes, plane_words * 4ull);
+        place(at_big, big, h->b_summ, sizeof(Summ) * summ_slots);
+        place(at_big, big, h->b_dlab, 2ull * dlab);
+        place(at_big, big, h->b_lab, 2ull * labels);
+        place(at_big, big, h->b_pw, 4ull * pwwords);
+        place(at_big, big, h->b_gplanes, 4ull * gwords);
+        place(at_big, big, h->b_gplanes2, 4ull * gwords2);
+        return ensure(h, h->b_big, big);
+    };
+    if (!ensure(h, h->b_small, small)) return CZ_ECUDA;
+    if (!place_big()) {
+        if (!dlab) return CZ_ECUDA;
+        dlab = plan_dense_labels(h, 0);                   // the dense scan runs without them, as the device's memory is short
+        if (!place_big()) return CZ_ECUDA;
+        h->err.clear();
+    }
     for (auto &x : at_small) x.first->p = static_cast<char *>(h->b_small.p) + x.second;
     for (auto &x : at_big) x.first->p = static_cast<char *>(h->b_big.p) + x.second;
     h->flags = flags;

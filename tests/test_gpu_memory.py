@@ -1,0 +1,57 @@
+"""Device memory: what a call allocates stays inside its plane budget, and a call
+that can do with less runs where memory is short."""
+import dataclasses
+
+import pytest
+
+from rabung_atlas32_b200 import sieve
+
+pytestmark = pytest.mark.gpu
+
+
+def rows(c, ps, mode):
+    out, _, _ = c.raw(ps, mode=mode, a4=False)
+    return [(o.p, o.r, o.M, o.L, o.witness, o.K) for o in out]
+
+
+@pytest.fixture(scope="module")
+def tuned():
+    from rabung_atlas32_b200.census import Census
+    with Census() as c:
+        yield c.tuning
+
+
+def test_dense_labels_inside_the_plane_budget(tuned):
+    """100 primes near 2^24 keep 0.77 GB of labels where the budget allows."""
+    from rabung_atlas32_b200.census import Census
+    ps = sieve.primes_from(1 << 24, 100)
+    with Census() as c:
+        want = rows(c, ps, "dense")
+    with Census(tuning=dataclasses.replace(tuned, plane_budget_mb=64)) as c:
+        rows(c, ps[:1], "dense")                          # static tables and small buffers are there
+        before = c.mem_info()[0]
+        assert rows(c, ps, "dense") == want
+        assert before - c.mem_info()[0] < (64 + 32) << 20
+    with Census(tuning=dataclasses.replace(tuned, plane_budget_mb=4)) as c:
+        assert rows(c, ps[:20], "dense") == want[:len(rows(c, ps[:20], "dense"))]      # no prime's labels fit
+
+
+def test_dense_scan_where_labels_do_not_fit_the_device(tuned):
+    """All but 0.5 GB of the device is taken; the labels of 300 primes near 2^24
+    would take 2 GiB."""
+    import torch
+    from rabung_atlas32_b200.census import Census
+    ps = sieve.primes_from(1 << 24, 300)
+    with Census() as c:
+        want = rows(c, ps, "auto")
+    with Census(tuning=tuned) as c:
+        rows(c, ps[:1], "dense")
+        torch.cuda.empty_cache()
+        free = c.mem_info()[0]
+        hold = torch.empty(free - (512 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            assert rows(c, ps, "dense") == want
+            assert rows(c, ps[:5], "auto") == want[:len(rows(c, ps[:5], "auto"))]      # the next call is not affected
+        finally:
+            del hold
+            torch.cuda.empty_cache()
