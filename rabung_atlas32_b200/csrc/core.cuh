@@ -359,9 +359,48 @@ u32 group_apex(const GroupDesc &G) {
     return (u32)(G.D * h / std::sqrt(h * h + (double)G.E * G.E));
 }
 
+// rows before the wide row groups of G
+u32 group_narrow_rows(const GroupDesc &G) {
+    return std::min(group_narrow_end(G.t, G.F), (G.D / G_ROWS + 1u) * G_ROWS);
+}
+
+// plane words of a profile on its own planes (a multiple of 8: vector loads and
+// tile copies align)
+u64 own_words(const PrimeDesc &P, const ProfDesc &D) {
+    return ((u64)D.npp * (P.nwords + P.nwords2) + 7ull) & ~7ull;
+}
+
+// Where the groups would take more than the plane budget, those that take more
+// than their members' own planes are dissolved: a full group takes less, one of
+// four members up to five times as much (2 B words a plane against 3 B / 32 a
+// member and stored plane), a whole call of scattered primes up to 1.9 times as
+// measured.  The waves of a call are cut by own planes, so the rest fits.
+void keep_groups_in_budget(CZ_HANDLE *h) {
+    u64 rest = 0, total = 0;                     // words of the profiles outside groups, of everything
+    std::vector<u64> took(h->hgroups.size()), own(h->hgroups.size(), 0);
+    for (const ProfDesc &D : h->hprof)
+        if (h->hp[D.prime].route == 2u) rest += own_words(h->hp[D.prime], D);
+    for (size_t g = 0; g < took.size(); ++g) {
+        GroupDesc G = h->hgroups[g];
+        group_layout(G, group_narrow_rows(G));
+        took[g] = (6ull * G.CL + G.nq) * G.np;
+        for (u32 k = 0; k < G.n; ++k) {
+            const ProfDesc &D = h->hprof[G.prof[k]];
+            own[g] += own_words(h->hp[D.prime], D);
+        }
+        rest -= own[g];
+        total += took[g];
+    }
+    if (4u * (total + rest) <= (u64)h->cfg.plane_budget_mb << 20) return;
+    size_t kept = 0;
+    for (size_t g = 0; g < took.size(); ++g)
+        if (took[g] <= own[g]) h->hgroups[kept++] = h->hgroups[g];
+    h->hgroups.resize(kept);
+}
+
 // row groups and items of one group; appended to rgs
 u32 group_items(GroupDesc &G, std::vector<RowGroup> &rgs) {
-    const u32 dn = std::min(group_narrow_end(G.t, G.F), (G.D / G_ROWS + 1u) * G_ROWS);
+    const u32 dn = group_narrow_rows(G);
     group_layout(G, dn);
     G.rg0 = (u32)rgs.size();
     u32 item = 0;
@@ -478,18 +517,20 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
             G.B = B; G.E = E; G.D = Dd; G.q = q; G.t = t; G.s = q - t + 1u;
             G.n = (u32)(e - i);
             G.nq = (u32)(std::upper_bound(primes_below.begin(), primes_below.end(), B) - primes_below.begin());
-            for (size_t k = i; k < e; ++k) {
-                ProfDesc &D = h->hprof[v[k]];
-                const pw_t p = h->hp[D.prime].p;
-                D.grouped = 1u;
-                D.qspec = q;
-                G.prof[k - i] = v[k];
-                G.job[k - i] = need_labels(h, D.prime, G.nq);
-                if ((u64)((p - 1u) >> 1) % r != 0u) G.sig |= 1u << (k - i);
-            }
+            for (size_t k = i; k < e; ++k) G.prof[k - i] = v[k];
             h->hgroups.push_back(G);
         }
     }
+    keep_groups_in_budget(h);
+    for (GroupDesc &G : h->hgroups)
+        for (u32 k = 0; k < G.n; ++k) {
+            ProfDesc &D = h->hprof[G.prof[k]];
+            const pw_t p = h->hp[D.prime].p;
+            D.grouped = 1u;
+            D.qspec = G.q;
+            G.job[k] = need_labels(h, D.prime, G.nq);
+            if ((u64)((p - 1u) >> 1) % G.r != 0u) G.sig |= 1u << k;
+        }
     u32 items = 0, own = 0;
     const GroupDesc *pv = nullptr;
     for (GroupDesc &G : h->hgroups) {
@@ -627,8 +668,8 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
         if (P.route != 2u || D.grouped) continue;
         // with B from the largest cap a denominator bound exists for every order
         if (!cover_D(P.p, P.B, D.Q, D.D)) { h->err = "no cover for p = " + std::to_string(P.p); return CZ_EINVAL; }
-        D.plane_off = plane_words;                      // multiple of 8 words: vector loads and tile copies align
-        plane_words += ((u64)D.npp * (P.nwords + P.nwords2) + 7ull) & ~7ull;
+        D.plane_off = plane_words;
+        plane_words += own_words(P, D);
         if (h->h_sidx.empty() || h->h_sidx.back() != D.prime) h->h_sidx.push_back(D.prime);
         D.local = (u32)h->h_sidx.size() - 1u;
         h->h_slist.push_back(g);

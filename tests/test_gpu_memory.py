@@ -55,3 +55,21 @@ def test_dense_scan_where_labels_do_not_fit_the_device(tuned):
         finally:
             del hold
             torch.cuda.empty_cache()
+
+
+def test_scattered_groups_inside_the_plane_budget(tuned):
+    """Ten windows of 10 primes, a factor of 2 apart: groups of 4 to 10 members,
+    which take up to four times their members' own planes."""
+    from rabung_atlas32_b200.census import Census
+    ps = [p for k in range(10) for p in sieve.primes_from(4200000000 >> k, 10)]
+    with Census(tuning=tuned) as c:
+        need = c.plane_bytes(ps, mode="sparse") >> 20
+        want = rows(c, ps, "sparse")
+        assert c.last_stats["kernels"] > 10               # groups were formed
+    with Census(tuning=dataclasses.replace(tuned, plane_budget_mb=need + 1)) as c:
+        rows(c, ps[:1], "sparse")
+        before = c.mem_info()[0]
+        assert rows(c, ps, "sparse") == want
+        assert c.last_stats["waves"] == 1
+        # planes, the labels beside them (a sixteenth) and the buffers' slack of a quarter
+        assert before - c.mem_info()[0] < need * 1.4 * 2 ** 20
