@@ -298,7 +298,7 @@ u64 plan_dense_labels(CZ_HANDLE *h, u64 limit) {
 
 // host plan of one call
 constexpr u32 CZ_NOSPEC = 1u << 16;      // internal: plan without speculative thresholds
-constexpr u32 CZ_NOGROUP = 1u << 17;     // internal: every sparse profile on its own planes (serving)
+constexpr u32 CZ_HOSTPLAN = 1u << 17;    // internal: host plan only, every sparse profile on its own planes (serving)
 
 // Cost of a profile on its own planes, in groups of its order and size (a group
 // costs the same whatever its members), and of a group besides its anchors, as
@@ -661,7 +661,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
     h->ndense = (u32)h->h_didx.size();
     h->nchunks = h->h_chunk.back();
     u64 gwords = 0, gwords2 = 0, pwwords = 0;
-    if (h->nsparse && !(flags & (CZ_NOSPEC | CZ_NOGROUP))) plan_groups(h, static_tables().primes, gwords, gwords2, pwwords);
+    if (h->nsparse && !(flags & (CZ_NOSPEC | CZ_HOSTPLAN))) plan_groups(h, static_tables().primes, gwords, gwords2, pwwords);
     for (u32 g = 0; g < h->nprof; ++g) {
         ProfDesc &D = h->hprof[g];
         const PrimeDesc &P = h->hp[D.prime];
@@ -711,6 +711,7 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
         return CZ_EINVAL;
     }
     h->dense_smem = max_slots_d * (u32)(sizeof(pw_t) + 2u) + 16u;
+    if (flags & CZ_HOSTPLAN) return CZ_OK;
     // device memory: uploaded descriptors, then the results (counters, records,
     // A4, states) that come back in one copy, in one buffer; tables in another
     size_t small = 0, big = 0;

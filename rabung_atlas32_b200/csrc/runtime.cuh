@@ -114,6 +114,7 @@ struct Held {
 constexpr u32 SRV_CAP_PRIMES = 1u << 20;       // resident primes
 constexpr u32 SRV_CAP_PROFILES = 1u << 22;     // resident profiles
 constexpr u32 SRV_CAP_SLOTS = 1u << 16;        // requests in flight
+constexpr u64 SRV_AUX_MB = 512;                // planes of a wave on the second handle: 285 primes near 2^32, 40 ms of filter
 constexpr int SRV_MIN_LAUNCH_US = 5000;        // a launch runs this long before it yields to arrivals
 // Requests of at most SRV_DIRECT_MS of modelled filter time run directly, in
 // calls of at most SRV_CALL_MS, one call a window (a prime near 2^32 takes about
@@ -407,7 +408,7 @@ void sieve_requests(cz_server *s, const std::vector<CzRequest *> &batch) {
     uint64_t total = 0;
     for (CzRequest *r : batch)
         if (!r->given && !r->sieved) { rs.push_back(r); lo.push_back(r->lo); cnt.push_back(r->count); total += r->count; }
-    if (rs.empty() || total > (1ull << 28)) return;
+    if (rs.empty() || total > (1ull << 24)) return;     // each by itself: the buffer lies outside the arena
     std::vector<uint32_t> got(total), found(rs.size(), 0u);
     if (cz_sieve(s->aux, lo.data(), cnt.data(), (uint32_t)rs.size(), got.data(), found.data())) return;
     size_t off = 0;
@@ -476,7 +477,7 @@ void admit(cz_server *s) {
         if (!back.empty()) { back.push_back(r); continue; }
         u32 mode = r->flags & CZ_AUTO;
         if (!mode) mode = CZ_AUTO;
-        int rc = plan(s->aux, r->primes.data(), n, mode | CZ_NOGROUP);
+        int rc = plan(s->aux, r->primes.data(), n, mode | CZ_HOSTPLAN);
         if (rc) { finish(s, r, rc, s->aux->err); continue; }
         // the resident (sparse) part of the plan
         std::vector<PrimeDesc> hp;
@@ -772,9 +773,10 @@ int cz_server_open(const cz_config *cfg, uint32_t slots, uint64_t slot_budget_by
     cz_server *s = new cz_server();
     if (cfg) s->cfg = *cfg; else cz_default_config(&s->cfg);
     const u64 per = slot_budget_bytes ? slot_budget_bytes : ((u64)s->cfg.plane_budget_mb << 20);
-    // the second handle's waves (oversize requests) hold at most one slot's planes
+    // the second handle's waves (joint calls, oversize requests) hold at most one
+    // slot's planes and SRV_AUX_MB: they live in the 4 GiB left beside the arena
     cz_config acfg = s->cfg;
-    acfg.plane_budget_mb = (uint32_t)std::max<u64>(64, std::min<u64>(acfg.plane_budget_mb, per >> 20));
+    acfg.plane_budget_mb = (uint32_t)std::max<u64>(64, std::min<u64>({acfg.plane_budget_mb, per >> 20, SRV_AUX_MB}));
     int rc = cz_open(&s->cfg, &s->h);
     if (!rc) rc = cz_open(&acfg, &s->aux);
     if (rc) { server_free(s); return rc; }

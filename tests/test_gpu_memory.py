@@ -73,3 +73,22 @@ def test_scattered_groups_inside_the_plane_budget(tuned):
         assert c.last_stats["waves"] == 1
         # planes, the labels beside them (a sixteenth) and the buffers' slack of a quarter
         assert before - c.mem_info()[0] < need * 1.4 * 2 ** 20
+
+
+def test_server_whose_arena_takes_the_device(tuned):
+    """An arena capped by the free memory leaves 4 GiB beside it.  In these: two
+    requests of 34,000 primes near 2^24, which run in one joint call, and one of
+    4096 primes near 2^32, which stays resident."""
+    from rabung_atlas32_b200.census import Census
+    from rabung_atlas32_b200.serving import Server
+    reqs = [(1 << 24, 34000), (15_000_000, 34000), (4_200_000_000, 4096)]
+    srv = Server(slots=16, slot_budget_mb=24 * 1024, tuning=tuned)
+    try:
+        ids = [srv.submit(lo, n) for lo, n in reqs]
+        got = [srv.fetch(rid, n) for rid, (lo, n) in zip(ids, reqs)]
+    finally:
+        srv.close()
+    with Census(tuning=tuned) as c:
+        for (lo, n), (primes, recs) in zip(reqs, got):
+            assert primes == sieve.primes_from(lo, n)
+            assert [(r.p, v.r, v.M, v.L, v.witness, v.K) for r in recs for v in r.profiles] == rows(c, primes, "auto")
