@@ -60,19 +60,25 @@ typedef struct cz_config {
     uint32_t sparse_min_p;   /* CZ_AUTO routes p >= this to the anchor filter */
     uint32_t cover_n;        /* cover shape: D ~ 2 sqrt(p/H) / cover_n (2..8) */
     uint32_t q_cap[10];      /* cover window Q per order r (index r), 3..255 */
-    uint32_t anchor_bits;    /* anchor length: 32 r^-(t-1) <= 2^-anchor_bits */
+    uint32_t anchor_bits;    /* anchor length: 32 r^-(t-1) <= 2^-anchor_bits (*) */
     uint32_t screen;         /* 1: bilateral screen after the anchor filter */
-    uint32_t sparse_blocks;  /* persistent filter grid (0: 2 per SM) */
+    uint32_t sparse_blocks;  /* most CTAs of the persistent filter (0: as many as are resident) */
     uint32_t use_graph;      /* 1: replay device work through a captured CUDA graph */
-    uint32_t cta_per_profile; /* CTAs sharing one profile's rows (L2 working set) */
-    uint32_t epoch_rows;     /* filter rows d per threshold epoch (0: 1024; at most 2^20) */
+    uint32_t cta_per_profile; /* CTAs sharing one profile's rows (L2 working set) (*) */
+    uint32_t epoch_rows;     /* filter rows d per threshold epoch (0: 1024; at most 2^20) (*) */
     uint32_t speculate;      /* 1: speculative thresholds floor(log_r p - margin), re-run on a miss */
     uint32_t spec_margin10[10];  /* margin per order r, in tenths */
-    uint32_t plane_budget_mb;    /* plane pool per wave; larger batches run as consecutive waves */
+    uint32_t plane_budget_mb;    /* plane pool per wave; larger batches run as consecutive waves; the
+                                    labels a dense scan keeps take at most as much (and 2 GiB) */
     uint32_t dense_steps;        /* dense scan segment: 32 x dense_steps values of x per warp */
-    uint32_t anchor_t[10];       /* anchor stages per order r (index r), 2..32; 0: from anchor_bits */
+    uint32_t anchor_t[10];       /* anchor stages per order r (index r), 2..32; 0: from anchor_bits (*) */
     uint32_t reserved[1];
 } cz_config;
+/* (*) profiles filtered by themselves: calls of few primes, calls without
+ * speculation, requests that stay resident in a server, and what is left over
+ * of larger calls.  Profiles filtered in groups of up to 32 take their stages
+ * from a cost model and have one threshold for all rows.  No field changes a
+ * record. */
 
 typedef struct cz_stats {
     float ms_setup, ms_table, ms_sparse, ms_dense, ms_a4, ms_finalize, ms_device;

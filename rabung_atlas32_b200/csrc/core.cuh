@@ -876,7 +876,9 @@ int enqueue(CZ_HANDLE *h, bool timed, u32 &launches) {
         fa.planes = P<u32>(h->b_gplanes);
         fa.planes2 = P<u32>(h->b_gplanes2);
         fa.next = P<u32>(h->b_counter) + 4;
-        gfilter_kernel<<<std::min(fa.nitems, (u32)h->sms), (G_WARPS + 2) * 32, G_SMEM, st>>>(fa);
+        fa.screen = h->cfg.screen;
+        const u32 most = h->cfg.sparse_blocks ? std::min(h->cfg.sparse_blocks, (u32)h->sms) : (u32)h->sms;
+        gfilter_kernel<<<std::min(fa.nitems, most), (G_WARPS + 2) * 32, G_SMEM, st>>>(fa);
         ++launches;
     }
     if (h->nsl) {
