@@ -4,12 +4,13 @@
 
 Searches, by coordinate descent from the defaults, the knobs that set how the
 work is cut and scheduled:
-  * anchor filter: anchor length policy (anchor_bits, then stages per order
-    r, anchor_t), cover window cap and speculation margin per order r, CTAs per profile
-    (cta_per_profile: CTAs sharing one profile's work items), rows per
-    threshold epoch (epoch_rows),
-    cover shape (cover_n: table radius vs rows), on a sample of the block below
-    2^32;
+  * anchor filter, on a sample of the block below 2^32: cover shape (cover_n:
+    table radius vs rows), cover window cap and speculation margin per order r;
+    and, in calls without speculation, where every profile is filtered by
+    itself (a grouped profile reads none of these): anchor length policy
+    (anchor_bits, then stages per order r, anchor_t), CTAs per profile
+    (cta_per_profile: CTAs sharing one profile's work items) and rows per
+    threshold epoch (epoch_rows);
   * dense scan: segment length (dense_steps, x per warp task), on primes near
     2^22;
   * routing: the dense/sparse crossover p (sparse_min_p).
@@ -80,18 +81,22 @@ def tune(quick: bool = False, log=print) -> dict:
     top = sieve.primes_ending(4294967291, 512 if quick else 1024)
     ref_ms, ref = _measure(base, top, "sparse")
     log(f"baseline sparse {ref_ms:.1f} ms")
+
+    def own(t):
+        return _measure(dataclasses.replace(t, speculate=0), top, "sparse")
+
     best = dataclasses.replace(base)
-    best_ms = ref_ms
-    space = {"anchor_bits": [3, 4, 5], "cta_per_profile": [1, 2, 3, 4], "epoch_rows": [256, 512, 1024, 2048],
-             "cover_n": [3, 4]}
-    rejected = []
+    best_ms, rec = own(best)
+    log(f"baseline without speculation {best_ms:.1f} ms")
+    space = {"anchor_bits": [3, 4, 5], "cta_per_profile": [1, 2, 3, 4], "epoch_rows": [256, 512, 1024, 2048]}
+    rejected = [] if rec == ref else [{"speculate": 0}]
     for _ in range(1 if quick else 2):
         for knob, values in space.items():
             for v in values:
                 if getattr(best, knob) == v:
                     continue
                 t = dataclasses.replace(best, **{knob: v})
-                ms, recs = _measure(t, top, "sparse")
+                ms, recs = own(t)
                 if recs != ref:
                     rejected.append({knob: v})
                     continue
@@ -107,13 +112,26 @@ def tune(quick: bool = False, log=print) -> dict:
             at = list(best.anchor_t)
             at[r] = v
             t = dataclasses.replace(best, anchor_t=tuple(at))
-            ms, recs = _measure(t, top, "sparse")
+            ms, recs = own(t)
             if recs != ref:
                 rejected.append({"anchor_t": r, "t": v})
                 continue
             log(f"  anchor_t[{r}]={v}: {ms:.1f} ms")
             if ms < best_ms * 0.995:
                 best, best_ms = t, ms
+    # cover shape, with speculation from here on
+    best_ms, _ = _measure(best, top, "sparse")
+    for v in (3, 4):
+        if best.cover_n == v:
+            continue
+        t = dataclasses.replace(best, cover_n=v)
+        ms, recs = _measure(t, top, "sparse")
+        if recs != ref:
+            rejected.append({"cover_n": v})
+            continue
+        log(f"  cover_n={v}: {ms:.1f} ms")
+        if ms < best_ms * 0.99:
+            best, best_ms = t, ms
     # cover window cap per order r: q never exceeds it, and the largest cap of
     # a prime's orders sets its table radius
     for r in range(2, 10):
