@@ -1176,7 +1176,7 @@ int census_impl(CZ_HANDLE *h, const pw_t *primes, uint32_t n, uint32_t flags, CZ
     cudaEventElapsedTime(&s.ms_h2d, h->ev[9], h->ev[10]);
     cudaEventElapsedTime(&s.ms_d2h, h->ev[6], h->ev[11]);
     read_times(h, &s);
-    s.d2h_bytes = sizeof(OutRecord) * h->nprof + ((flags & CZ_A4) ? 4ull * n : 0ull);
+    s.d2h_bytes = h->down_bytes;
     s.n_primes = n; s.n_dense = h->ndense; s.n_sparse = h->nsparse; s.n_profiles = h->nprof;
     s.kernels = launches;
     const OutRecord *ho = reinterpret_cast<const OutRecord *>(got(h->b_out));
@@ -1236,6 +1236,8 @@ int census_impl(CZ_HANDLE *h, const pw_t *primes, uint32_t n, uint32_t flags, CZ
         s.n_fallback += s2.n_fallback;
         s.ms_respec = s2.ms_device + s2.ms_respec;
         s.kernels += s2.kernels;
+        s.h2d_bytes += s2.h2d_bytes;
+        s.d2h_bytes += s2.d2h_bytes;
         h->sub_live = true;
         h->have_plan = h->have_plan && h->sub->have_plan;
     }
@@ -1253,6 +1255,8 @@ int census_impl(CZ_HANDLE *h, const pw_t *primes, uint32_t n, uint32_t flags, CZ
         for (size_t k = 0; k < fb_p.size(); ++k)
             for (u32 j = 0; j < popc(fb_mask[k]); ++j) out[fb_first[k] + j] = tmp[t++];
         s.n_fallback += (u32)fb.size();
+        s.h2d_bytes += s2.h2d_bytes;
+        s.d2h_bytes += s2.d2h_bytes;
         h->have_plan = false;   // the plan now describes the fallback batch
     }
     h->last = s;
