@@ -52,8 +52,9 @@ class Tuning:
 def _as_u32_array(values):
     n = len(values)
     if n:
-        try:                              # integers in range: converted in C
-            return (ctypes.c_uint32 * n).from_buffer(array.array("I", values))
+        try:                              # integers in range: converted in C (bytes: by value, not as words)
+            ints = list(values) if isinstance(values, (bytes, bytearray)) else values
+            return (ctypes.c_uint32 * n).from_buffer(array.array("I", ints))
         except (TypeError, OverflowError):
             pass
     arr = (ctypes.c_uint32 * n)()
@@ -66,7 +67,7 @@ def _as_u32_array(values):
 
 def to_records(primes, out, a4v) -> list:
     """codec.Record list from C records grouped by prime in input order."""
-    ps = np.array(primes, dtype=np.int64)
+    ps = np.array(primes if isinstance(primes, (list, tuple, np.ndarray)) else list(primes), dtype=np.int64)
     admissible = ((ps[:, None] - 1) % np.arange(2, 10) == 0).sum(axis=1) * (ps > 2)
     ends = np.cumsum(admissible).tolist()
     fields = np.frombuffer(out, dtype=out._type_)[:ends[-1] if ends else 0]
