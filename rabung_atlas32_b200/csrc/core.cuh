@@ -307,7 +307,10 @@ constexpr u32 CZ_HOSTPLAN = 1u << 17;    // internal: host plan only, every spar
 // a cost of 1/8, 1/5, 1/3 41.2 / 36.7 / 36.7 ms; 37 primes near 7e8 with 1/8,
 // 1/5, 1/3 2.32 / 2.21 / 1.99 ms on the device, 7 primes near 4.2e9 1.99 / 2.13 /
 // 2.93 ms: the line lies between.
-constexpr double OWN_COST = 1.0 / 4.0, GROUP_FIXED = 2e7;
+#ifndef CZ_GROUP_OWN_COST
+#define CZ_GROUP_OWN_COST (1.0 / 4.0)
+#endif
+constexpr double OWN_COST = CZ_GROUP_OWN_COST, GROUP_FIXED = 2e7;
 
 // compared planes and anchor stages of a group: least cost per visited anchor
 // and position of the row.  A stage costs F loads; beta is the bits it is worth
