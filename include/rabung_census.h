@@ -61,7 +61,7 @@ typedef struct cz_config {
     uint32_t cover_n;        /* cover shape: D ~ 2 sqrt(p/H) / cover_n (2..8) */
     uint32_t q_cap[10];      /* cover window Q per order r (index r), 3..255 */
     uint32_t anchor_bits;    /* anchor length: 32 r^-(t-1) <= 2^-anchor_bits (*) */
-    uint32_t screen;         /* 1: bilateral screen after the anchor filter */
+    uint32_t screen;         /* 1: bilateral screen after the anchor filter; 0: none, and no groups (*) */
     uint32_t sparse_blocks;  /* most CTAs of the persistent filter (0: as many as are resident) */
     uint32_t use_graph;      /* 1: replay device work through a captured CUDA graph */
     uint32_t cta_per_profile; /* CTAs sharing one profile's rows (L2 working set) (*) */
@@ -75,7 +75,7 @@ typedef struct cz_config {
     uint32_t reserved[1];
 } cz_config;
 /* (*) profiles filtered by themselves: calls of few primes, calls without
- * speculation, requests that stay resident in a server, and what is left over
+ * speculation or screen, requests that stay resident in a server, and what is left over
  * of larger calls.  Profiles filtered in groups of up to 32 take their stages
  * from a cost model and have one threshold for all rows.  No field changes a
  * record. */

@@ -456,7 +456,6 @@ struct GFilterArgs {
     u32 ngroups, nitems;
     const u32 *planes, *planes2;
     u32 *next;                    // work counter
-    u32 screen;                   // 0: survivors are completed without the screen
 };
 
 struct GCand { u32 b, dm; };      // numerator; d << 5 | member
@@ -695,7 +694,7 @@ __device__ __noinline__ u32 gscreen_batch(const GShared &sh, const GroupDesc &G,
             const GEnt e = w.scr[n + lane];
             b = e.b;
             d = e.d;
-            keep = sh.a.screen ? gscreen<F>(G, sh.a.planes + G.off, sh.a.planes2 + G.off2, b, d, e.alive) : e.alive;
+            keep = gscreen<F>(G, sh.a.planes + G.off, sh.a.planes2 + G.off2, b, d, e.alive);
         }
         for (u32 bal = __ballot_sync(0xFFFFFFFFu, keep != 0u); bal; bal = __ballot_sync(0xFFFFFFFFu, keep != 0u)) {
             if (keep) {

@@ -1,5 +1,6 @@
-"""Tuning fields that act on the grouped filter too: the screen and the number of
-CTAs.  The records stay."""
+"""Tuning fields that act also in calls whose profiles would be filtered in groups:
+the screen (without it there are no groups) and the number of CTAs.  The records
+stay."""
 import dataclasses
 
 import pytest
@@ -17,7 +18,7 @@ def run(tuning, ps):
         return [(o.p, o.r, o.M, o.L, o.witness, o.K) for o in out], st
 
 
-def test_screen_and_sparse_blocks_act_on_groups():
+def test_screen_and_sparse_blocks_act():
     """64 times one prime: two full groups of every order, nothing beside them."""
     from rabung_atlas32_b200.census import Census
     with Census() as c:
