@@ -69,7 +69,7 @@ typedef struct cz_config {
     uint32_t speculate;      /* 1: speculative thresholds floor(log_r p - margin), re-run on a miss */
     uint32_t spec_margin10[10];  /* margin per order r, in tenths */
     uint32_t plane_budget_mb;    /* plane pool per wave; larger batches run as consecutive waves; the
-                                    labels a dense scan keeps take at most as much (and 2 GiB) */
+                                    labels a dense scan keeps take at most what is left of it, and 2 GiB */
     uint32_t dense_steps;        /* dense scan segment: 32 x dense_steps values of x per warp */
     uint32_t anchor_t[10];       /* anchor stages per order r (index r), 2..32; 0: from anchor_bits (*) */
     uint32_t reserved[1];
@@ -199,7 +199,7 @@ int cz_census_interval(cz_handle *h, uint64_t lo, uint64_t hi, uint32_t flags, u
  * a profile whose speculative threshold missed is re-run there without
  * speculation, as cz_census does (records are unchanged by it).  A request
  * whose colour planes exceed the server's whole plane budget runs on the
- * second handle in waves of at most one slot's planes; a caller's non-prime is
+ * second handle in waves of at most one slot's planes and 1 GiB; a caller's non-prime is
  * refused before any device work.  A refusal reaches only the request that
  * caused it.  Submit and poll may be
  * called from any host thread.  The reference has no serving path; the

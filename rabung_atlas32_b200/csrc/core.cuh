@@ -159,14 +159,14 @@ bool ensure(CZ_HANDLE *h, Buf &b, size_t bytes) {
     if (b.p) cudaFree(b.p);
     b.p = nullptr;
     b.cap = 0;
+    cudaError_t e = cudaSuccess;
     for (size_t want : {bytes + bytes / 4, bytes}) {       // no slack where memory is short
-        const cudaError_t e = cudaMalloc(&b.p, want);
+        e = cudaMalloc(&b.p, want);
         if (e == cudaSuccess) { b.cap = want; return true; }
         cudaGetLastError();                                // or the next launch check reports it
         b.p = nullptr;
-        ck(h, e, "cudaMalloc");
     }
-    return false;
+    return ck(h, e, "cudaMalloc");
 }
 
 template <class T> T *P(Buf &b) { return reinterpret_cast<T *>(b.p); }
@@ -255,8 +255,9 @@ u32 qspec_for(const cz_config &c, double lg_p, u32 r, bool allow, u32 level) {
 // 210 in memory (dense.cuh), in waves of at most DENSE_LABEL_WORDS 16-bit labels
 // (one prime below 2^33 takes 0.98e9 of them at most).  Where the line lies: 400
 // primes near 7e4 take 0.53 ms with the scan's own powers and 0.31 ms with kept
-// labels, 400 near 2e4 the same either way (0.39 ms).  The pool stays inside the
-// plane budget; a prime whose labels alone exceed it takes a power for every x.
+// labels, 400 near 2e4 the same either way (0.39 ms).  The pool stays inside what
+// the planes leave of the budget; a prime whose labels alone exceed that takes a
+// power for every x.
 // Returns the pool's size in labels (limit 0: no labels).
 constexpr u64 DENSE_LABEL_MIN_P = 1u << 16, DENSE_LABEL_WORDS = 1ull << 30;
 u64 plan_dense_labels(CZ_HANDLE *h, u64 limit) {
@@ -708,7 +709,8 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
         max_nq = (u32)(std::lower_bound(hs.begin(), hs.end(), nmax) - hs.begin());
     }
     h->lab_smem = max_slots_t * (u32)(sizeof(pw_t) + 2u) + 16u;
-    u64 dlab = plan_dense_labels(h, std::min(DENSE_LABEL_WORDS, ((u64)c.plane_budget_mb << 20) / 2u));
+    const u64 budget = (u64)c.plane_budget_mb << 20, planes = 4ull * (plane_words + gwords + gwords2 + pwwords);
+    u64 dlab = plan_dense_labels(h, std::min(DENSE_LABEL_WORDS, (budget - std::min(budget, planes)) / 2u));
     u64 labels = 0;
     for (LabelJob &J : h->hjobs) { J.off = labels; labels += (J.nq + 63u) & ~63u; }
     h->table_smem = max_slots_t * (u32)(sizeof(pw_t) + 2u) + 8u + max_nq * 2u + 16u;

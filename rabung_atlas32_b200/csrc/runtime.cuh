@@ -114,7 +114,7 @@ struct Held {
 constexpr u32 SRV_CAP_PRIMES = 1u << 20;       // resident primes
 constexpr u32 SRV_CAP_PROFILES = 1u << 22;     // resident profiles
 constexpr u32 SRV_CAP_SLOTS = 1u << 16;        // requests in flight
-constexpr u64 SRV_AUX_MB = 512;                // planes of a wave on the second handle: 285 primes near 2^32, 40 ms of filter
+constexpr u64 SRV_AUX_MB = 1024;               // planes and labels of a wave on the second handle (570 primes near 2^32)
 constexpr int SRV_MIN_LAUNCH_US = 5000;        // a launch runs this long before it yields to arrivals
 // Requests of at most SRV_DIRECT_MS of modelled filter time run directly, in
 // calls of at most SRV_CALL_MS, one call a window (a prime near 2^32 takes about

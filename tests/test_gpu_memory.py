@@ -92,3 +92,20 @@ def test_server_whose_arena_takes_the_device(tuned):
         for (lo, n), (primes, recs) in zip(reqs, got):
             assert primes == sieve.primes_from(lo, n)
             assert [(r.p, v.r, v.M, v.L, v.witness, v.K) for r in recs for v in r.profiles] == rows(c, primes, "auto")
+
+
+def test_planes_and_labels_share_the_budget(tuned):
+    """One call with 100 sparse primes near 2^28 and 100 dense ones near 2^24
+    (sparse_min_p between them): 0.05 GB of planes, 0.77 GB of labels."""
+    from rabung_atlas32_b200.census import Census
+    ps = sieve.primes_from(1 << 24, 100) + sieve.primes_from(1 << 28, 100)
+    t = dataclasses.replace(tuned, sparse_min_p=1 << 26)
+    with Census(tuning=t) as c:
+        want = rows(c, ps, "auto")
+        assert c.last_stats["n_dense"] == 100 and c.last_stats["n_sparse"] == 100
+        planes = c.plane_bytes(ps, mode="auto") >> 20
+    with Census(tuning=dataclasses.replace(t, plane_budget_mb=planes + 32)) as c:
+        rows(c, ps[:1], "dense")
+        before = c.mem_info()[0]
+        assert rows(c, ps, "auto") == want
+        assert before - c.mem_info()[0] < (planes + 32) * 1.4 * 2 ** 20 + (8 << 20)
