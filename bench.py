@@ -18,7 +18,9 @@ every prime, through the certified rational-anchor filter.  Metric: profiles/s.
             host;
   roofline  dominant kernel (gfilter_kernel): 32-bit words compared per second
             against what the shared-memory load path can deliver (32 words a
-            clock and SM at the maximum clock);
+            clock and SM at the maximum clock); two rows tested together load
+            their base words once, so 1/(2t) of the words compared (4 to 17 %,
+            t = 3..13 stages) are not loads;
   cpu_baseline / --impl reference
             the reference's own CPU sparse engines -- `target p c f 64 1 8192 1`
             for the coupled order pairs {2, 4} and {3, 6}, `advance adaptive
@@ -474,7 +476,8 @@ def main():
                 "peak": round(peak_words / 1e9, 2), "unit": "G words compared/s",
                 "frac": round(achieved / peak_words, 4), "traffic": None,
                 "algorithmic": f"{tests} words compared per call (visited anchors x stages x compared planes, counted "
-                               "in-kernel; the time includes the few profiles on sparse_kernel)",
+                               "in-kernel; 1/(2t) of them, base words shared by two rows, are loaded once for both; the "
+                               "time includes the few profiles on sparse_kernel)",
                 "launch_ms": round(ms_sparse, 3),
                 "peak_source": "32 words per clock and SM (128-byte shared-memory load path) at the maximum SM clock",
                 "alu_plane_tests_peak_per_s": peak_tests, "montgomery_peak_per_s": peak_mont,

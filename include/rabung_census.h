@@ -89,7 +89,7 @@ typedef struct cz_stats {
     uint32_t waves;                 /* consecutive waves the batch ran as */
     uint32_t kernels;               /* kernel launches of the call */
     uint64_t words, completions;    /* sparse filter words visited, exact completions */
-    uint64_t tests;                 /* plane-window comparisons executed by the filter */
+    uint64_t tests;                 /* plane words compared by the filter (anchors x stages x planes) */
     uint64_t h2d_bytes, d2h_bytes;  /* bytes copied each way, re-runs included */
     uint64_t staged_bytes;          /* colour-plane bytes the filter copied into shared memory */
 } cz_stats;
@@ -119,8 +119,9 @@ int cz_census(cz_handle *h, const uint32_t *primes, uint32_t n, uint32_t flags,
  * are checked; stats receives the device times. */
 int cz_replay(cz_handle *h, cz_stats *stats);
 
-/* Device memory the colour planes of these primes would take (admission
- * control for serving; no reference counterpart). */
+/* Device memory the colour planes of these primes take at most (the waves of a
+ * call and admission to a server are cut by it; full groups take less; labels of
+ * primes, about a sixteenth, come on top; no reference counterpart). */
 uint64_t cz_plane_bytes(const cz_handle *h, const uint32_t *primes, uint32_t n, uint32_t flags);
 
 /* Name and SM count of the handle's GPU (keys the autotuner's saved choices;
@@ -183,8 +184,9 @@ int cz_census_interval(cz_handle *h, uint64_t lo, uint64_t hi, uint32_t flags, u
                        uint32_t *n_profiles, uint32_t *a4_out, cz_stats *stats);
 
 /* ---- serving ---------------------------------------------------------------
- * A server runs requests of up to about 20 ms of filter time at once, together,
- * and keeps larger ones resident on the GPU until their records
+ * A server runs requests of up to about 20 ms of filter time in joint calls of
+ * up to 40 ms, one call between two stretches of the resident filter, and keeps
+ * larger ones resident on the GPU until their records
  * are final: the descriptors, per-profile state, colour planes, records and A4
  * of its primes live in device arrays sized when the server opens (colour
  * planes: slots x slot_budget_bytes, capped by free device memory), so a

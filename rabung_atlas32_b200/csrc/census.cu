@@ -5,8 +5,12 @@
 //   plan (host, O(n)): admissible orders, route (dense / sparse), cover
 //     (B, D_r, Q_r) by the integer certificate, plane and summary layout;
 //   setup_kernel: primality, Montgomery constants, roots of unity;
-//   table_kernel + sparse_kernel: signed planes, persistent anchor filter;
-//   dense_scan_kernel + dense_merge_kernel: exhaustive half-interval scan;
+//   plabel_kernel, gpack_kernel, gtable_*, gfilter_kernel: labels, bit-sliced
+//     planes and the anchor filter of profiles in groups of 32;
+//   table_kernel + sparse_kernel: signed planes and the anchor filter of the
+//     profiles left by themselves;
+//   dlabel_kernel + dense_scan_kernel + dense_merge_kernel: exhaustive
+//     half-interval scan;
 //   finalize_kernel: prefix, optional direct certification, K, records;
 //   a4_kernel: quadratic A4 counts.
 // The device work of the last call can be replayed on resident inputs

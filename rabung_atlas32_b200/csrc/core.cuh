@@ -449,8 +449,10 @@ u32 need_labels(CZ_HANDLE *h, u32 i, u32 nq) {
 // The sparse profiles of each order, in descending p, are cut into groups of up
 // to 32 and profiles kept on their own planes, at least modelled cost: a group
 // runs its largest prime's cover at its least threshold.  Cuts are considered
-// at 32 members and where p falls by more than 1/16 (a run of near primes is
-// best filled up).  Sets ProfDesc.grouped and the group's q as its members'
+// at 32 members and where p falls by more than 1/16: a run of near primes is
+// best filled up, and fewer cuts are less host work (1/8, 1/16 and 1/32 are the
+// same within 1 % on 40 windows of 61 primes, 200 of 12, 4000 scattered primes
+// and blocks).  Sets ProfDesc.grouped and the group's q as its members'
 // speculative threshold.
 void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords, u64 &gwords2, u64 &pwwords) {
     std::vector<u32> by[10];
@@ -504,7 +506,8 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
             const u32 q = best[e].q;
             const pw_t pmax = prime(i), pmin = prime(e - 1);
             // a cover serves every smaller prime too: neighbouring groups share one,
-            // and with it their row groups, while that costs less than 1/1024
+            // and with it their row groups, while that costs less than 1/1024 (1/128
+            // and 1/8192 are the same within 1 % on the same calls)
             u32 own = 0;
             for (size_t k = i; k < e; ++k) own = std::max(own, h->hp[h->hprof[v[k]].prime].B);
             if (q != cq || own > B || (u64)pmax + pmax / 1024u < (u64)cover_p) {

@@ -70,7 +70,8 @@ __device__ __forceinline__ u32 lookup_label(const pw_t *keys, const unsigned sho
     return 0xFFFFu;
 }
 
-// exact floor(x / r) for x < 2^16, r <= 9: multiply by ceil(2^32 / r)
+// x mod r by ceil(2^32 / r): the quotient is exact while x r < 2^32 (colours:
+// x < 2^16, r <= 9; sums of labels: x < 2^18, r = m <= 2520)
 CZ_HD u32 magic_of(u32 r) { return (u32)(((u64(1) << 32) + r - 1) / r); }
 CZ_HD u32 mod_small(u32 x, u32 r, u32 magic) { return x - r * umulhi(x, magic); }
 

@@ -4,8 +4,8 @@ A request asks for the profiles (and A4) of the `count` consecutive primes
 starting at `lo`.  `Server` drives the library's native serving runtime
 (cz_server_open / cz_submit / cz_next_done / cz_poll, csrc/runtime.cuh):
 
-  * a request of up to about 20 ms of filter time runs at once between
-    launches, together with the others like it in one call; a larger one stays
+  * a request of up to about 20 ms of filter time runs between launches,
+    together with others like it in a call of up to 40 ms; a larger one stays
     resident on the GPU (descriptors, state, colour planes, records) until its
     records are final; admission is by free
     colour-plane memory and descriptor space;
