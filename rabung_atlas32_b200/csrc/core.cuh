@@ -114,9 +114,15 @@ struct CZ_HANDLE {
         b_slist, b_dlist, b_dpre, b_out, b_a4, b_counter,
         b_dlab, b_dlaboff, b_dlabp, b_groups, b_rgs, b_item0, b_jobs, b_lab, b_pw, b_gplanes, b_gplanes2;
     // host copies of the current plan
-    std::vector<PrimeDesc> hp, hp_next;
+    std::vector<PrimeDesc> hp;
     std::vector<ProfDesc> hprof;
     std::vector<u32> h_chunk, h_summp, h_didx, h_sidx, h_slist, h_dlist;
+    // the lists of a plan in the making: a refused one leaves those above whole
+    struct Lists {
+        std::vector<PrimeDesc> hp;
+        std::vector<ProfDesc> hprof;
+        std::vector<u32> chunk, summp, didx, dlist;
+    } next;
     // dense scan: waves of primes whose label arrays fit the pool together
     struct DenseWave { u32 i0, i1, lchunk0, lchunks, chunk0, chunk1; };
     std::vector<u64> h_dlaboff;         // per dense-local prime (NO_LABELS: powers in the scan)
@@ -460,6 +466,23 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
         const ProfDesc &D = h->hprof[g];
         if (h->hp[D.prime].route == 2u && std::min(D.qspec, D.Q) >= 3u) by[D.r].push_back(g);
     }
+    // the members of a group that stays
+    auto join = [h](GroupDesc &G) {
+        for (u32 k = 0; k < G.n; ++k) {
+            ProfDesc &D = h->hprof[G.prof[k]];
+            const pw_t p = h->hp[D.prime].p;
+            D.grouped = 1u;
+            D.qspec = G.q;
+            G.job[k] = need_labels(h, D.prime, G.nq);
+            if ((u64)((p - 1u) >> 1) % G.r != 0u) G.sig |= 1u << k;
+        }
+    };
+    // could the groups exceed the budget at all?  At most 4 planes of 2 B words,
+    // guards and colours of the primes each, were every profile a group
+    u64 maxB = 0;
+    for (const PrimeDesc &P : h->hp) maxB = std::max<u64>(maxB, P.B);
+    const bool tight = 16ull * h->nprof * (2u * std::max<u64>(maxB, 16384u) + maxB / 2u + 8192u) >
+                       (u64)h->cfg.plane_budget_mb << 20;
     struct Cut { double cost; size_t from; u32 q; };
     for (u32 r = 9; r >= 2; --r) {                   // costliest orders first: the launch ends on cheap items
         auto &v = by[r];
@@ -525,19 +548,14 @@ void plan_groups(CZ_HANDLE *h, const std::vector<u32> &primes_below, u64 &gwords
             G.n = (u32)(e - i);
             G.nq = (u32)(std::upper_bound(primes_below.begin(), primes_below.end(), B) - primes_below.begin());
             for (size_t k = i; k < e; ++k) G.prof[k - i] = v[k];
+            if (!tight) join(G);
             h->hgroups.push_back(G);
         }
     }
-    keep_groups_in_budget(h);
-    for (GroupDesc &G : h->hgroups)
-        for (u32 k = 0; k < G.n; ++k) {
-            ProfDesc &D = h->hprof[G.prof[k]];
-            const pw_t p = h->hp[D.prime].p;
-            D.grouped = 1u;
-            D.qspec = G.q;
-            G.job[k] = need_labels(h, D.prime, G.nq);
-            if ((u64)((p - 1u) >> 1) % G.r != 0u) G.sig |= 1u << k;
-        }
+    if (tight) {
+        keep_groups_in_budget(h);
+        for (GroupDesc &G : h->hgroups) join(G);
+    }
     u32 items = 0, own = 0;
     const GroupDesc *pv = nullptr;
     for (GroupDesc &G : h->hgroups) {
@@ -579,68 +597,53 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
     const cz_config &c = h->cfg;
     const u32 mode = flags & CZ_AUTO;
     const u32 seg = dense_seg(c);
-    // primes, orders and routes first, beside the resident plan: a request
-    // refused here leaves that plan whole, for a replay
-    std::vector<PrimeDesc> &next = h->hp_next;
-    next.assign(n, PrimeDesc{});
-    u64 all_chunks = 0, all_slots = 0;
+    // primes, orders and routes beside the resident plan: a request refused in
+    // this loop leaves that plan whole, for a replay
+    CZ_HANDLE::Lists &N = h->next;
+    N.hp.assign(n, PrimeDesc{});
+    N.hprof.clear();
+    N.didx.clear(); N.dlist.clear(); N.summp.clear();
+    N.chunk.assign(1, 0u);
+    u64 plane_words = 0;
+    u32 max_slots_t = 8, max_slots_d = 8, max_nq = 0, nsparse = 0;
+    u64 summ_slots = 0;
     for (u32 i = 0; i < n; ++i) {
         const pw_t p = primes[i];
         if (p < 2u || (u64)p >= PW_LIMIT) { h->err = "prime out of domain: " + std::to_string(p); return CZ_EINVAL; }
-        PrimeDesc &P = next[i];
+        PrimeDesc &P = N.hp[i];
         P.p = p;
         P.mask = p > 2u ? mask_of(p) & (masks ? masks[i] : ~0u) : 0u;
+        P.m = lcm_of_mask(P.mask);
+        P.e = P.mask ? (p - 1u) / P.m : 0u;
+        P.first_prof = (u32)N.hprof.size();
         P.nprof = popc(P.mask);
         P.job = 0xFFFFFFFFu;
         if (!P.nprof) continue;
         P.route = route_of(c, p, P.mask, mode, P.B);
-        if (P.route == 2u) continue;
-        if (mode == CZ_SPARSE) {
-            h->err = "sparse path unsupported for p = " + std::to_string(p);
-            return CZ_EINVAL;
-        }
-        const u32 nch = dense_chunks(p, seg);
-        all_chunks += nch;
-        all_slots += (u64)nch * P.nprof;
-        if (all_chunks > 0xFFFFFFFFull || all_slots > 0xFFFFFFFFull) {
-            h->err = "dense scan too large for one call (chunk index beyond 32 bits)";
-            return CZ_ELIMIT;
-        }
-    }
-    h->have_plan = false;
-    h->hp.swap(next);
-    h->hprof.clear();
-    h->h_didx.clear(); h->h_sidx.clear(); h->h_slist.clear(); h->h_dlist.clear();
-    h->h_chunk.assign(1, 0u); h->h_summp.clear();
-    h->hgroups.clear(); h->hrgs.clear(); h->hitem0.clear(); h->hjobs.clear();
-    h->nsparse = 0; h->gmaxB = 0; h->gmaxq = 0;
-    u64 plane_words = 0;
-    u32 max_slots_t = 8, max_slots_d = 8, max_nq = 0;
-    u64 summ_slots = 0;
-    for (u32 i = 0; i < n; ++i) {
-        PrimeDesc &P = h->hp[i];
-        const pw_t p = P.p;
-        P.m = lcm_of_mask(P.mask);
-        P.e = P.mask ? (p - 1u) / P.m : 0u;
-        P.first_prof = (u32)h->hprof.size();
-        if (!P.nprof) continue;
         const bool sparse = P.route == 2u;
-        const u32 B = P.B;
         if (sparse) {
             // view widths in words, multiples of 4: every view and every tile
             // copy of the filter starts on a 16-byte boundary
-            P.K0 = (B + 31u) / 32u + 4u;
+            P.K0 = (P.B + 31u) / 32u + 4u;
             P.nwords = (2u * P.K0 + 8u + 3u) & ~3u;
-            P.K2 = (B + 63u) / 64u + 4u;
+            P.K2 = (P.B + 63u) / 64u + 4u;
             P.nwords2 = (2u * P.K2 + 8u + 3u) & ~3u;
-            ++h->nsparse;
+            ++nsparse;
             max_slots_t = std::max(max_slots_t, hash_slots(P.m));
         } else {
+            if (mode == CZ_SPARSE) {
+                h->err = "sparse path unsupported for p = " + std::to_string(p);
+                return CZ_EINVAL;
+            }
             const u32 nch = dense_chunks(p, seg);
-            h->h_didx.push_back(i);
-            h->h_summp.push_back((u32)summ_slots);
+            if ((u64)N.chunk.back() + nch > 0xFFFFFFFFull || summ_slots + (u64)nch * P.nprof > 0xFFFFFFFFull) {
+                h->err = "dense scan too large for one call (chunk index beyond 32 bits)";
+                return CZ_ELIMIT;
+            }
+            N.didx.push_back(i);
+            N.summp.push_back((u32)summ_slots);
             summ_slots += (u64)nch * P.nprof;
-            h->h_chunk.push_back(h->h_chunk.back() + nch);
+            N.chunk.push_back(N.chunk.back() + nch);
             max_slots_d = std::max(max_slots_d, hash_slots(P.m));
         }
         const double lg_p = sparse ? std::log((double)p) : 0.0;
@@ -651,18 +654,25 @@ int plan(CZ_HANDLE *h, const pw_t *primes, u32 n, u32 flags, const u32 *masks = 
             D.r = r;
             D.np = planes_for(r);
             D.npp = planes_stored(r);
-            D.out_slot = (u32)h->hprof.size();
+            D.out_slot = (u32)N.hprof.size();
             if (sparse) {
                 D.Q = q_for(c, r);
                 D.qspec = qspec_for(c, lg_p, r, !(flags & CZ_NOSPEC), level);
                 D.tpref = c.anchor_t[r] ? c.anchor_t[r] : anchor_pref(r, c.anchor_bits);
             } else {
-                D.local = (u32)h->h_didx.size() - 1u;
-                h->h_dlist.push_back((u32)h->hprof.size());
+                D.local = (u32)N.didx.size() - 1u;
+                N.dlist.push_back((u32)N.hprof.size());
             }
-            h->hprof.push_back(D);
+            N.hprof.push_back(D);
         }
     }
+    h->have_plan = false;
+    h->hp.swap(N.hp);
+    h->hprof.swap(N.hprof);
+    h->h_didx.swap(N.didx); h->h_dlist.swap(N.dlist); h->h_summp.swap(N.summp); h->h_chunk.swap(N.chunk);
+    h->h_sidx.clear(); h->h_slist.clear();
+    h->hgroups.clear(); h->hrgs.clear(); h->hitem0.clear(); h->hjobs.clear();
+    h->nsparse = nsparse; h->gmaxB = 0; h->gmaxq = 0;
     h->n = n;
     h->nprof = (u32)h->hprof.size();
     h->ndense = (u32)h->h_didx.size();
